@@ -7,7 +7,9 @@ The op names, argument order, shapes and error behaviour follow the reference's 
   * CPU tensors go through the host-pointer entries (the library copies to the device, runs, copies back), exactly
     what the reference's host extension does through its dlopen seam;
   * CUDA tensors go through the `_dev` entries on torch's current stream: nothing is allocated or synchronised by the
-    library, the result tensor is allocated by torch.
+    library, the result tensor is allocated by torch.  The calls of a decode or prefill step take one native function each
+    (`_native`, csrc/qb_torch.cpp), which returns None for a call it does not serve: the Python path below it then
+    converts the arguments or raises.
 
 There is no CPU arm here: a missing library or CUDA device is an error, never a silent fallback.
 """
@@ -18,6 +20,7 @@ import ctypes as C
 import torch
 
 from . import _lib
+from ._lib import native as _native
 from .formats import QuantType, kquant_geometry  # noqa: F401
 
 __all__ = [
@@ -107,6 +110,9 @@ def gguf_vecdot(blocks, x, qtype: int):
 
 def gguf_vecdot_rows(blocks, x, n: int, k: int, qtype: int, force_generic: bool = False):
     """Raw-block GEMV with m >= 1 shared activation rows: x [m,k] -> fp32 [m,n] (CUDA tensors)."""
+    out = _native.vecdot_rows(blocks, x, n, k, qtype, force_generic)
+    if out is not None:
+        return out
     g = _geom(qtype)
     _u8(blocks, "blocks", 2)
     _check(n > 0 and k > 0 and k % 256 == 0, "n must be positive and k a positive multiple of 256")
@@ -127,6 +133,9 @@ def gguf_vecdot_rows(blocks, x, n: int, k: int, qtype: int, force_generic: bool 
 
 def gguf_vecdot_dense(blocks, x, n: int, k: int, qtype: int):
     """Dense decode GEMV: blocks [n*k/256,type_size], one activation x fp16/fp32 [1,k] -> fp32 [1,n]."""
+    out = _native.vecdot_dense(blocks, x, n, k, qtype)
+    if out is not None:
+        return out
     g = _geom(qtype)
     _u8(blocks, "blocks", 2)
     _check(x.dim() == 2 and x.shape[0] == 1 and x.shape[1] == k, "x must be fp16/fp32 [1,k]")
@@ -151,6 +160,9 @@ def gguf_vecdot_dense2(blocks_a, blocks_b, x, n_a: int, n_b: int, k: int, qtype:
     """Two dense decode GEMVs that share their activation, in one launch (additive; a layer's gate and up projections):
     blocks_a [n_a*k/256,type_size], blocks_b [n_b*k/256,type_size], x fp16/fp32 [1,k] -> (fp32 [1,n_a], fp32 [1,n_b]).
     Device tensors only."""
+    out = _native.vecdot_dense2(blocks_a, blocks_b, x, n_a, n_b, k, qtype)
+    if out is not None:
+        return out
     g = _geom(qtype)
     _u8(blocks_a, "blocks_a", 2)
     _u8(blocks_b, "blocks_b", 2)
@@ -215,6 +227,9 @@ def gguf_vecdot_moe(blocks, x, row_offsets, qtype: int):
 
 def gguf_dequantize(blocks, qtype: int):
     """Raw blocks [rows,type_size] -> fp16 [rows,256], bit-exact half(dl*q - ml)."""
+    out = _native.dequantize(blocks, qtype)
+    if out is not None:
+        return out
     g = _geom(qtype)
     _u8(blocks, "blocks", 2)
     _check(blocks.shape[1] == g.block_bytes, f"this format's raw GGUF block is {g.block_bytes} bytes, got {blocks.shape[1]}")
@@ -567,6 +582,9 @@ def _scale_first(a, low, high, scale, zero, row_offsets, qtype, grouped):
 
 def gguf_gemv_scale_first(a, low, high, scale, zero, qtype: int):
     """Dense GEMV over a resident `gguf_prepare_gemv` artifact -> fp16 [rows,n]."""
+    out = _native.gemv_scale_first(a, low, high, scale, zero, qtype)
+    if out is not None:
+        return out
     return _scale_first(a, low, high, scale, zero, None, qtype, False)
 
 
@@ -612,6 +630,9 @@ def _bc(a, low, high, units, row_offsets, qtype, grouped):
 
 def gguf_gemv_bc(a, low, high, units, qtype: int):
     """CUDA-core GEMV over the merged form: Native code planes plus packed scale units -> fp32 [1,n]."""
+    out = _native.gemv_bc(a, low, high, units, qtype)
+    if out is not None:
+        return out
     return _bc(a, low, high, units, None, qtype, False)
 
 
@@ -628,6 +649,9 @@ def gemv_plane(a, low, high, scale, zero, bits_lo: int, bits_hi: int, group_size
     dense when row_offsets is None (E == 1), else ragged with cumulative int32 offsets.  Returns [rows,n] in a's dtype
     unless out_dtype (torch.float16 / bfloat16 / float32) says otherwise.  Passing max_rows (an upper bound on any
     expert's row count) skips the host-side validation of a device-resident row_offsets, which would synchronise."""
+    out = _native.gemv_plane(a, low, high, scale, zero, bits_lo, bits_hi, group_size, code_offset, row_offsets, out_dtype, max_rows)
+    if out is not None:
+        return out
     _check(a.is_cuda and a.dim() == 2 and a.dtype in (torch.float16, torch.bfloat16), "a must be a CUDA fp16/bf16 [rows,k] tensor")
     _u8(low, "low", 3)
     e, n, k = low.shape[0], low.shape[1], a.shape[1]
@@ -673,6 +697,10 @@ def gemm_plane(a, low, high, scale, zero, bits_lo: int, bits_hi: int, group_size
 
     split_k selects the decode form: 128 x 128 tiles with shallow rings and K split over that many slices (0 = as many
     as fill the SMs, at most 8; 1 = shallow rings only) whose fp32 partial planes a second small kernel sums."""
+    if split_k is None:
+        out = _native.gemm_plane(a, low, high, scale, zero, bits_lo, bits_hi, group_size, code_offset, row_offsets)
+        if out is not None:
+            return out
     _check(a.is_cuda and a.dim() == 2 and a.dtype in (torch.float16, torch.bfloat16), "a must be a CUDA fp16/bf16 [rows,k] tensor")
     _u8(low, "low", 3)
     e, n, k = low.shape[0], low.shape[1], a.shape[1]
@@ -762,6 +790,9 @@ def _fq_common(a, low, high, units, g, grouped):
 
 def gguf_dense_fully_quantized(a, low, high, units, qtype: int):
     """Dense GEMM reading the format's own packed scale bytes (planes + units) -> fp16 [m,n]."""
+    out = _native.dense_fully_quantized(a, low, high, units, qtype)
+    if out is not None:
+        return out
     g = _geom(qtype)
     e, n, k = _fq_common(a, low, high, units, g, False)
     _check(e == 1, "dense artifact must have one expert dimension")

@@ -124,3 +124,29 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = h
     return _lib
+
+
+class _Native:
+    """The CPython binding of the device-tensor calls (_native.so), loaded and bound to `lib()` on first use; afterwards
+    its functions are plain attributes of this object."""
+
+    def __getattr__(self, name):
+        if name.startswith("__"):
+            raise AttributeError(name)
+        import importlib.machinery
+        import importlib.util
+        import torch  # noqa: F401  -- its libraries have to be loaded first
+        path = os.path.join(_HERE, "_native.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is not built. Build it with:  python -m quactlize_b200.build")
+        h = lib()
+        full = __package__ + "._native"
+        loader = importlib.machinery.ExtensionFileLoader(full, path)
+        m = importlib.util.module_from_spec(importlib.util.spec_from_file_location(full, path, loader=loader))
+        loader.exec_module(m)
+        m.bind({n: C.cast(getattr(h, n), C.c_void_p).value for n in m.entries()})
+        self.__dict__.update({k: v for k, v in vars(m).items() if not k.startswith("__")})
+        return self.__dict__[name]
+
+
+native = _Native()

@@ -1,6 +1,10 @@
 """Build libquactlize_b200.so in-tree with nvcc for sm_100a (no torch types; a plain C-ABI shared library).
 
     python -m quactlize_b200.build [-v] [--force]
+
+and, beside it, quactlize_b200/_native.so: the CPython binding of the device-tensor calls (csrc/qb_torch.cpp, host code only,
+compiled with g++ against torch's headers and linked to torch's libraries).
+
     python -m quactlize_b200.build --variant NAME --define MACRO[=VALUE] [--define ...]
 
 Each .cu is compiled to an object only when it or a header changed, then linked into
@@ -29,6 +33,35 @@ LIB = os.path.join(CSRC, "libquactlize_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
          "--expt-relaxed-constexpr", "-I", os.path.join(os.path.dirname(HERE), "include")]
+
+
+NATIVE_SRC = os.path.join(CSRC, "qb_torch.cpp")
+NATIVE = os.path.join(HERE, "_native.so")
+
+
+def build_native(verbose: bool = False, force: bool = False) -> str:
+    """The CPython binding; rebuilt when its source or the C-ABI header changed."""
+    header = os.path.join(os.path.dirname(HERE), "include", "quactlize_b200.h")
+    newest = max(os.path.getmtime(NATIVE_SRC), os.path.getmtime(header))
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest:
+        return NATIVE
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    includes = [*cpp_extension.include_paths(), os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"),
+                sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{i}" for i in includes], NATIVE_SRC,
+           "-o", NATIVE, f"-L{libdir}", f"-Wl,-rpath,{libdir}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch",
+           "-lc10_cuda", "-lc10"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return NATIVE
 
 
 def sources():
@@ -63,8 +96,10 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
         if (verbose or ptxas_info) and (r.stdout or r.stderr):
             print(r.stdout + r.stderr, flush=True)
 
-    with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)) + 1)) as ex:
+        native = ex.submit(build_native, verbose, force)
         list(ex.map(run, jobs))
+        native.result()
     if jobs or not os.path.exists(LIB):
         run([NVCC, "-shared", "-o", LIB, *objs, "-cudart", "shared"])
     return LIB
