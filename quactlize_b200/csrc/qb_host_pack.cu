@@ -14,8 +14,14 @@
 // byte-identical copies and every consumer here (GEMV and GEMM) reads Native planes.
 #include <cuda_fp16.h>
 
+#include <emmintrin.h>
+#include <sched.h>
+
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "qb_kquant.cuh"
@@ -35,72 +41,173 @@ template <int Bits> inline int plane_get(uint8_t const* plane, int64_t logical) 
   return (plane[bit >> 3] >> (bit & 7)) & ((1 << Bits) - 1);
 }
 
-template <int QT>
-void pack_unit_sb(uint8_t const* block, uint8_t* sb) {
-  using F = kq::Fmt<QT>;
-  using U = kq::Unit<QT>;
-  std::memset(sb, 0, U::kSbBytes);
-  sb[0] = block[F::kD]; sb[1] = block[F::kD + 1];
-  if constexpr (F::kHasMin) { sb[2] = block[F::kDmin]; sb[3] = block[F::kDmin + 1]; }
-  for (int g = 0; g < F::kGroups; ++g) {
-    int sc, mn;
-    kq::scale_min<QT>(block + F::kScaleOff, g, sc, mn);
-    kq::put_bits(sb, U::bit_of(g, 0), F::kScaleBits, sc + F::kScaleBias);
-    if constexpr (F::kHasMin) kq::put_bits(sb, U::bit_of(g, 1), F::kMinBits, mn);
+// ---- work split -----------------------------------------------------------------------------------------------------------
+//
+// The producers are independent per output row, so rows are dealt to host threads in contiguous runs.  A thread costs about
+// 30 us to start and join and packs about 3 GB/s (bound by the byte work, not by memory), so it is given at least 512 KB of
+// raw blocks; more than 16 gain nothing (memory and page faults of the fresh outputs bound it then).  One 14336 x 4096 Q4_K
+// matrix: 66 ms a code at a time on one thread, 10 ms with the vector forms below, 1.5 ms of those on 16 threads.
+int host_threads(int64_t bytes) {
+  int cpus = int(std::thread::hardware_concurrency());
+  cpu_set_t set;
+  if (sched_getaffinity(0, sizeof(set), &set) == 0) cpus = CPU_COUNT(&set);
+  return int(std::max<int64_t>(1, std::min<int64_t>(std::min(16, cpus), bytes / (512 << 10))));
+}
+
+// fn(first, last) over [0, rows), rows cut at multiples of `step`
+template <class Fn>
+void for_rows(int64_t rows, int64_t step, int64_t bytes, Fn const& fn) {
+  int64_t const units = (rows + step - 1) / step;
+  int const nt = int(std::min<int64_t>(host_threads(bytes), units));
+  auto part = [&](int t) {
+    int64_t const r0 = units * t / nt * step, r1 = std::min(rows, units * (t + 1) / nt * step);
+    if (r0 < r1) fn(r0, r1);
+  };
+  std::vector<std::thread> pool;
+  int started = 1;
+  try {
+    for (; started < nt; ++started) pool.emplace_back(part, started);
+  } catch (std::system_error const&) {}                     // no more threads: the rest runs here
+  part(0);
+  for (int t = started; t < nt; ++t) part(t);
+  for (auto& th : pool) th.join();
+}
+
+// ---- one superblock ---------------------------------------------------------------------------------------------------------
+//
+// The fields of consecutive code bytes belong to consecutive elements, so a run of 32 bytes shifted and masked is a run of 32
+// codes, squeezed to 4, 2 or 1 bits each with SSE2 (part of every x86-64).
+
+inline __m128i load16(uint8_t const* p) { return _mm_loadu_si128(reinterpret_cast<__m128i const*>(p)); }
+inline __m128i pair4(__m128i v, int shift) {                              // 16-bit lanes: two 4-bit codes -> one byte
+  v = _mm_srli_epi16(v, shift);
+  return _mm_or_si128(_mm_and_si128(v, _mm_set1_epi16(0x0F)), _mm_and_si128(_mm_srli_epi16(v, 4), _mm_set1_epi16(0xF0)));
+}
+inline void squeeze4(uint8_t const* src, int shift, uint8_t* dst) {       // 32 codes of 4 bits -> 16 bytes
+  _mm_storeu_si128(reinterpret_cast<__m128i*>(dst), _mm_packus_epi16(pair4(load16(src), shift), pair4(load16(src + 16), shift)));
+}
+inline __m128i quad2(__m128i v, int shift) {                              // 32-bit lanes: four 2-bit codes -> one byte
+  v = _mm_and_si128(_mm_srli_epi32(v, shift), _mm_set1_epi8(3));
+  v = _mm_or_si128(v, _mm_srli_epi32(v, 6));
+  return _mm_and_si128(_mm_or_si128(v, _mm_srli_epi32(v, 12)), _mm_set1_epi32(0xFF));
+}
+inline void squeeze2(uint8_t const* src, int shift, uint8_t* dst) {       // 32 codes of 2 bits -> 8 bytes
+  __m128i const w = _mm_packs_epi32(quad2(load16(src), shift), quad2(load16(src + 16), shift));
+  _mm_storel_epi64(reinterpret_cast<__m128i*>(dst), _mm_packus_epi16(w, w));
+}
+inline void squeeze1(uint8_t const* src, int shift, uint8_t* dst) {       // 32 codes of 1 bit -> 4 bytes
+  for (int i = 0; i < 2; ++i) {                                           // the bit moves to the top of its byte
+    uint16_t const m = uint16_t(_mm_movemask_epi8(_mm_slli_epi16(load16(src + 16 * i), 7 - shift)));
+    std::memcpy(dst + 2 * i, &m, 2);
   }
 }
 
 template <int QT>
-int pack_units(uint8_t const* blocks, uint8_t* units, int n, int k, int experts) {
+void planes_sb(uint8_t const* b, uint8_t* low, uint8_t* high) {           // 256 codes, offset-binary
+  for (int c = 0; c < 8; ++c) {                                           // 32 elements at a time
+    if constexpr (QT == 12 || QT == 13) {
+      squeeze4(b + (QT == 12 ? 16 : 48) + 32 * (c >> 1), 4 * (c & 1), low + 16 * c);
+      if constexpr (QT == 13) squeeze1(b + 16, c, high + 4 * c);
+    } else if constexpr (QT == 14) {
+      int const h = c >> 2, n = (c >> 1) & 1, q = c & 1;
+      squeeze4(b + 64 * h + 32 * q, 4 * n, low + 16 * c);
+      squeeze2(b + 128 + 32 * h, 2 * q + 4 * n, high + 8 * c);
+    } else {
+      int const h = c >> 2, t = c & 3;
+      squeeze2(b + (QT == 11 ? 32 : 16) + 32 * h, 2 * t, low + 8 * c);
+      if constexpr (QT == 11) squeeze1(b, t + 4 * h, high + 4 * c);       // a set mask bit is code bit 2 of the biased code
+    }
+  }
+}
+
+template <int QT>
+void pack_unit_sb(uint8_t const* block, uint8_t* sb) {
   using F = kq::Fmt<QT>;
   using U = kq::Unit<QT>;
-  int64_t const nsb = k / 256;
-  if (nsb % U::kSbPerUnit) return 24;
+  sb[0] = block[F::kD]; sb[1] = block[F::kD + 1];
+  if constexpr (F::kHasMin) { sb[2] = block[F::kDmin]; sb[3] = block[F::kDmin + 1]; }
+  if constexpr (QT == 14) {
+    std::memcpy(sb + 2, block + F::kScaleOff, 16);                        // int8 sub-scales as they are
+  } else {
+    uint8_t* dst = sb + U::kHdr;
+    int sc[F::kGroups], mn[F::kGroups];
+    for (int g = 0; g < F::kGroups; ++g) kq::scale_min<QT>(block + F::kScaleOff, g, sc[g], mn[g]);
+    constexpr int kPiece = U::kRun * F::kScaleBits > 48 ? U::kRun / 2 : U::kRun;       // fields that share a 64-bit word
+    auto put = [&](int const* v, int bias) {
+      for (int p = 0; p < U::kRun; p += kPiece) {
+        uint64_t w = 0;
+        for (int i = 0; i < kPiece; ++i) w |= uint64_t(uint32_t(v[p + i] + bias)) << (F::kScaleBits * i);
+        std::memcpy(dst, &w, kPiece * F::kScaleBits / 8);
+        dst += kPiece * F::kScaleBits / 8;
+      }
+    };
+    static_assert(!F::kHasMin || F::kMinBits == F::kScaleBits, "scales and mins are fields of one width");
+    for (int r = 0; r < F::kGroups; r += U::kRun) {
+      put(sc + r, F::kScaleBias);
+      if constexpr (F::kHasMin) put(mn + r, 0);
+    }
+  }
+}
+
+constexpr int kColTile = 32;      // rows walked side by side: their units and scale-plane entries are neighbours in memory
+
+template <int QT>
+void pack_units_rows(uint8_t const* blocks, uint8_t* units, int n, int64_t nsb, int64_t r0, int64_t r1) {
+  using F = kq::Fmt<QT>;
+  using U = kq::Unit<QT>;
   int64_t const nu = nsb / U::kSbPerUnit;
-  for (int e = 0; e < experts; ++e)
-    for (int col = 0; col < n; ++col)
-      for (int64_t sb = 0; sb < nsb; ++sb)
-        pack_unit_sb<QT>(blocks + ((int64_t(e) * n + col) * nsb + sb) * F::kBytes,
-                         units + ((int64_t(e) * nu + sb / U::kSbPerUnit) * n + col) * U::kUnitTotal +
-                             (sb % U::kSbPerUnit) * U::kSbBytes);
+  for (int64_t t0 = r0; t0 < r1; t0 += kColTile)
+    for (int64_t sb = 0; sb < nsb; ++sb)
+      for (int64_t r = t0; r < std::min(r1, t0 + kColTile); ++r)
+        pack_unit_sb<QT>(blocks + (r * nsb + sb) * F::kBytes,
+                         units + ((r / n * nu + sb / U::kSbPerUnit) * n + r % n) * U::kUnitTotal + (sb % U::kSbPerUnit) * U::kSbBytes);
+}
+
+template <int QT>
+int pack_units(uint8_t const* blocks, uint8_t* units, int n, int k, int experts) {
+  using U = kq::Unit<QT>;
+  int64_t const nsb = k / 256, rows = int64_t(experts) * n;
+  if (nsb % U::kSbPerUnit) return 24;
+  for_rows(rows, kColTile, rows * nsb * kq::Fmt<QT>::kBytes,
+           [&](int64_t r0, int64_t r1) { pack_units_rows<QT>(blocks, units, n, nsb, r0, r1); });
   return 0;
 }
 
-// planes (+ optional fp16 planes) from raw blocks
+// raw blocks -> planes, with the packed units and / or the fp16 planes beside them (nullptr: not wanted)
 template <int QT>
-void raw_to_planes(uint8_t const* blocks, uint8_t* low, uint8_t* high, uint16_t* scale, uint16_t* zero,
-                   int n, int k, int experts) {
+int raw_to_planes(uint8_t const* blocks, uint8_t* low, uint8_t* high, uint8_t* units, uint16_t* scale, uint16_t* zero,
+                  int n, int k, int experts) {
   using F = kq::Fmt<QT>;
-  constexpr int G = F::kGroups, GS = 256 / G;
-  int64_t const nsb = k / 256;
-  std::memset(low, 0, size_t(experts) * n * k * F::kLo / 8);
-  if (F::kHi && high) std::memset(high, 0, size_t(experts) * n * k * F::kHi / 8);
-  int64_t const scale_k = nsb * G;
-  for (int e = 0; e < experts; ++e)
-    for (int col = 0; col < n; ++col)
-      for (int64_t sb = 0; sb < nsb; ++sb) {
-        uint8_t const* blk = blocks + ((int64_t(e) * n + col) * nsb + sb) * F::kBytes;
-        float const d = h2f(kq::load_u16(blk + F::kD));
-        float const dmin = F::kHasMin ? h2f(kq::load_u16(blk + F::kDmin)) : 0.f;
-        for (int g = 0; g < G; ++g) {
-          int sc, mn;
-          kq::scale_min<QT>(blk + F::kScaleOff, g, sc, mn);
-          for (int j = 0; j < GS; ++j) {
-            int const u = kq::code<QT>(blk, g, j) + F::kCodeBias;
-            int64_t const logical = (int64_t(e) * n + col) * k + sb * 256 + g * GS + j;
-            plane_put<F::kLo>(low, logical, u);
-            if constexpr (F::kHi != 0) plane_put<(F::kHi ? F::kHi : 1)>(high, logical, u >> F::kLo);
-          }
+  using U = kq::Unit<QT>;
+  constexpr int G = F::kGroups;
+  int64_t const nsb = k / 256, nu = nsb / U::kSbPerUnit, rows = int64_t(experts) * n, scale_k = nsb * G;
+  if (units && nsb % U::kSbPerUnit) return 24;
+  for_rows(rows, kColTile, rows * nsb * F::kBytes, [&](int64_t r0, int64_t r1) {
+    for (int64_t t0 = r0; t0 < r1; t0 += kColTile)
+      for (int64_t sb = 0; sb < nsb; ++sb)
+        for (int64_t r = t0; r < std::min(r1, t0 + kColTile); ++r) {
+          uint8_t const* blk = blocks + (r * nsb + sb) * F::kBytes;
+          planes_sb<QT>(blk, low + (r * nsb + sb) * (32 * F::kLo), F::kHi ? high + (r * nsb + sb) * (32 * F::kHi) : nullptr);
+          if (units)
+            pack_unit_sb<QT>(blk, units + ((r / n * nu + sb / U::kSbPerUnit) * n + r % n) * U::kUnitTotal +
+                                      (sb % U::kSbPerUnit) * U::kSbBytes);
           if (scale) {
-            // scale = half(dl), zero = half(-ml), then the offset-binary bias folded in float and rounded once
-            uint16_t const s = f2h(d * float(sc));
-            uint16_t const z0 = f2h(-(dmin * float(mn)));
-            uint16_t const z = f2h(h2f(z0) - float(F::kCodeBias) * h2f(s));
-            int64_t const dst = (int64_t(e) * scale_k + sb * G + g) * n + col;
-            scale[dst] = s; zero[dst] = z;
+            float const d = h2f(kq::load_u16(blk + F::kD));
+            float const dmin = F::kHasMin ? h2f(kq::load_u16(blk + F::kDmin)) : 0.f;
+            for (int g = 0; g < G; ++g) {
+              int sc, mn;
+              kq::scale_min<QT>(blk + F::kScaleOff, g, sc, mn);
+              // scale = half(dl), zero = half(-ml), then the offset-binary bias folded in float and rounded once
+              uint16_t const s = f2h(d * float(sc));
+              uint16_t const z0 = f2h(-(dmin * float(mn)));
+              uint16_t const z = f2h(h2f(z0) - float(F::kCodeBias) * h2f(s));
+              int64_t const dst = (r / n * scale_k + sb * G + g) * n + r % n;
+              scale[dst] = s; zero[dst] = z;
+            }
           }
         }
-      }
+  });
+  return 0;
 }
 
 template <int QT>
@@ -196,10 +303,7 @@ extern "C" int quactlize_ppu_prepare_fully_quantized_v1(uint8_t const* blocks, u
                                                          int n, int k, int experts, int qtype) {
   if (!blocks || !low || !units || experts <= 0 || !shape_ok(n, k)) return 20;
   if ((qtype == 11 || qtype == 13 || qtype == 14) && !high) return 21;
-#define EXPR ((k / 256) % kq::Unit<Q>::kSbPerUnit ? 24 : (raw_to_planes<Q>(blocks, low, high, nullptr, nullptr, n, k, experts), \
-                                                       pack_units<Q>(blocks, units, n, k, experts)))
-  QT_DISPATCH(qtype, EXPR, 22)
-#undef EXPR
+  QT_DISPATCH(qtype, raw_to_planes<Q>(blocks, low, high, units, nullptr, nullptr, n, k, experts), 22)
 }
 
 extern "C" int quactlize_ppu_recover_fully_quantized_v1(uint8_t const* low, uint8_t const* high, uint8_t const* units,
@@ -214,7 +318,7 @@ extern "C" int quactlize_b200_prepare_gemv(uint8_t const* blocks, uint8_t* low, 
                                             uint16_t* zero, int n, int k, int experts, int qtype) {
   if (!blocks || !low || !scale || !zero || experts <= 0 || n <= 0 || k <= 0 || k % 256) return 20;
   if ((qtype == 11 || qtype == 13 || qtype == 14) && !high) return 21;
-  QT_DISPATCH(qtype, (raw_to_planes<Q>(blocks, low, high, scale, zero, n, k, experts), 0), 22)
+  QT_DISPATCH(qtype, raw_to_planes<Q>(blocks, low, high, nullptr, scale, zero, n, k, experts), 22)
 }
 
 // Placement entries: the placement of this library is the Native order, so both directions are copies.
