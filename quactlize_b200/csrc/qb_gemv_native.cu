@@ -390,6 +390,11 @@ int enqueue_native_gemv(uint8_t const* blocks, __half const* x, float* out, int 
   a.status = rt_device_status_ptr();
   int const rows_hint = offsets ? max_rows : m_rows;
   bool const aligned = (reinterpret_cast<uintptr_t>(blocks) % 16 == 0) && (reinterpret_cast<uintptr_t>(x) % 16 == 0);
+  static int const kr_mode = [] { char const* v = std::getenv("QB_KR"); return v ? std::atoi(v) : 3; }();
+  bool const kr = !per_row_x && !force_generic && a.status;
+  if (kr && (kr_mode & 4 || (kr_mode & 1 && !offsets && m_rows >= 2) || (kr_mode & 2 && offsets))) {
+    if (enqueue_kq_rows(blocks, x, out, offsets, n, bpr, a.experts, m_rows, qtype, a.status, stream)) return 0;
+  }
   // several activation rows per weight pass: the tensor-core kernel (QUACTLIZE_B200_Q4K_SMALLM=off keeps the CUDA-core ones)
   static bool const no_mma = [] { char const* v = std::getenv("QUACTLIZE_B200_Q4K_SMALLM"); return v && v[0] == 'o'; }();
   bool const batch = offsets ? m_rows >= 2 * a.experts : m_rows >= 2;
@@ -426,6 +431,7 @@ int enqueue_native_gemv(uint8_t const* blocks, __half const* x, float* out, int 
     // the other four formats: the single-row kernel once per activation row (rows after the first hit L2)
     if (enqueue_kquant_gemv1(blocks, x, out, offsets, n, bpr, a.experts, m_rows, max_rows, qtype, a.status, stream)) return 0;
   }
+  if (kr && enqueue_kq_rows(blocks, x, out, offsets, n, bpr, a.experts, m_rows, qtype, a.status, stream)) return 0;
   if (per_row_x) {
     a.mtiles = 1;
     launch_generic_qt<1>(qtype, a, 1, stream);

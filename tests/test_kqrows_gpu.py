@@ -1,0 +1,62 @@
+"""Raw-block kernel for several activation rows (csrc/qb_gemv_kqrows.cu) at the edges of its tiles, passes and alignments.
+
+Its operands are exact (fp16 activations, sub-scale x code products of at most 11 bits), so what is left is the fp32
+accumulation of the tensor cores: at most a few units of 2^-23 of the sum of the terms' sizes, which for K normal terms
+is about sqrt(K)/3 times the largest output: 2e-5 of the largest output at K = 16384.
+"""
+import numpy as np
+import pytest
+import torch
+
+import quactlize_b200 as qb
+from oracle import kquant as kq
+from quactlize_b200 import synth
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+QTYPES = (10, 11, 12, 13, 14)
+
+
+def _cuda(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+
+
+# (rows, n, k): one tile and its edges, every split of the warps and of K (passes, clusters), K whose rows end off a
+# 16-byte boundary, activation rows at and beyond one group of eight
+@pytest.mark.parametrize("m,n,k", [(2, 16, 256), (3, 17, 512), (8, 15, 1280), (5, 130, 2304), (9, 48, 1024), (4, 2500, 1024),
+                                   (7, 333, 4096), (2, 1000, 4352), (8, 600, 14336), (6, 5000, 5376), (1, 77, 768), (3, 40, 33024)])
+@pytest.mark.parametrize("qt", QTYPES)
+def test_rows(qt, m, n, k):
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=qt + m)
+    x = synth.activations(m, k, seed=n)
+    out = qb.gguf_vecdot_rows(_cuda(blocks), _cuda(x), n, k, qt).cpu().numpy()
+    ref = np.concatenate([kq.vecdot_dense(blocks, x[i:i + 1], n, k, qt).reshape(1, n) for i in range(m)])
+    fp16_sums = m <= 2 and (qt in (12, 13) or k // 256 % 8 == 0)     # the one-row kernels
+    assert kq.max_rel(out, ref) < (4e-3 if fp16_sums else 2e-5)
+
+
+@pytest.mark.parametrize("counts", [[0, 0, 1, 0], [3, 0, 17, 8, 1], [1] * 16, [0, 9, 0, 0, 0, 0, 2]])
+@pytest.mark.parametrize("n,k", [(70, 768), (300, 2304), (40, 8448)])
+@pytest.mark.parametrize("qt", QTYPES)
+def test_moe(qt, n, k, counts):
+    e, rows = len(counts), sum(counts)
+    blocks = synth.kquant_blocks(qt, e * n * k // 256, seed=qt).reshape(e, n * k // 256, -1)
+    x = synth.activations(rows, k, seed=3)
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    out = qb.gguf_vecdot_moe(_cuda(blocks), _cuda(x), _cuda(off), qt).cpu().numpy()
+    assert kq.max_rel(out, kq.vecdot_moe(blocks, x, off, n, k, qt)) < 2e-5
+
+
+@pytest.mark.parametrize("qt", QTYPES)
+def test_blocks_off_a_16_byte_boundary(qt):
+    """A view into a larger buffer: 16-byte formats need the plain kernel there, the others start mid-unit."""
+    m, n, k = 3, 40, 1024
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=qt)
+    x = synth.activations(m, k, seed=1)
+    want = np.concatenate([kq.vecdot_dense(blocks, x[i:i + 1], n, k, qt).reshape(1, n) for i in range(m)])
+    for shift in (2, 4, 8):
+        buf = torch.zeros(blocks.size + 64, dtype=torch.uint8, device=DEV)
+        view = buf[shift:shift + blocks.size].view(blocks.shape)
+        view.copy_(_cuda(blocks))
+        out = qb.gguf_vecdot_rows(view, _cuda(x), n, k, qt).cpu().numpy()
+        assert kq.max_rel(out, want) < 2e-5, shift
