@@ -91,6 +91,10 @@ int quactlize_b200_vecdot_dev_v1(uint8_t const* blocks, int64_t block_bytes, uin
 int quactlize_b200_vecdot_moe_dev_v1(uint8_t const* blocks, int64_t block_bytes, uint16_t const* x, int const* offsets,
                                      float* out, int n, int blocks_per_row, int experts, int total_rows, int max_rows,
                                      int qtype, void* stream);
+/* in bounds whatever `offsets` hold: may be enqueued before they are checked; 40 = not covered, use the entry above */
+int quactlize_b200_vecdot_moe_clamped_dev_v1(uint8_t const* blocks, int64_t block_bytes, uint16_t const* x, int const* offsets,
+                                             float* out, int n, int blocks_per_row, int experts, int total_rows, int qtype,
+                                             void* stream);
 int quactlize_b200_dequantize_dev_v1(uint8_t const* blocks, int64_t block_bytes, uint16_t* out, int n_blocks, int qtype,
                                      void* stream);
 int quactlize_b200_prepass_unit_dev_v1(uint8_t const* units, uint16_t* scale, uint16_t* zero, int n, int k, int experts,

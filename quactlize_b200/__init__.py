@@ -197,6 +197,9 @@ def _offsets_info(row_offsets, experts, total_rows):
 def gguf_vecdot_moe(blocks, x, row_offsets, qtype: int):
     """Ragged MoE decode over raw blocks: blocks [E,n*k/256,type_size], gathered x [rows,k], offsets int32 [E+1]
     -> fp32 [rows,n]."""
+    out = _native.vecdot_moe(blocks, x, row_offsets, qtype)
+    if out is not None:
+        return out
     g = _geom(qtype)
     _u8(blocks, "blocks", 3)
     _check(x.dim() == 2, "x must be fp16/fp32 [total_rows,k]")

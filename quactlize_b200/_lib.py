@@ -34,6 +34,7 @@ SIGNATURES = {
     "quactlize_b200_vecdot_dense2_dev_v1": (I, [P, I, P, I, I64, P, P, P, I, I, P]),
     "quactlize_b200_vecdot_rows_dev_v1": (I, [P, I64, P, P, I, I, I, I, I, P]),
     "quactlize_b200_vecdot_moe_dev_v1": (I, [P, I64, P, P, P, I, I, I, I, I, I, P]),
+    "quactlize_b200_vecdot_moe_clamped_dev_v1": (I, [P, I64, P, P, P, I, I, I, I, I, P]),
     "quactlize_b200_dequantize_dev_v1": (I, [P, I64, P, I, I, P]),
     "quactlize_b200_prepass_unit_dev_v1": (I, [P, P, P, I, I, I, I, I, P]),
     "quactlize_ppu_gemv_lowbit": (I, [P, P, P, P, P, P, I, I, I, I, I, I, P, I]),

@@ -150,6 +150,18 @@ extern "C" int quactlize_b200_vecdot_moe_dev_v1(uint8_t const* b, int64_t block_
   return rt_check_launch("raw-block MoE GEMV enqueue") ? 0 : kRuntimeError;
 }
 
+// The same launch through the one kernel that clamps the offsets to [0, total_rows] and their differences to >= 0: it stays in
+// bounds whatever they hold, so a caller may enqueue it before the offsets are checked.  40: a form it does not cover.
+extern "C" int quactlize_b200_vecdot_moe_clamped_dev_v1(uint8_t const* b, int64_t block_bytes, uint16_t const* x, int const* offsets,
+                                                        float* out, int n, int bpr, int experts, int total_rows, int qtype, void* stream) {
+  if (kq::raw_bytes(qtype) == 0) return 2;
+  if (block_bytes != kq::raw_bytes(qtype) || n <= 0 || bpr <= 0 || experts <= 0 || total_rows <= 0 || !b || !x || !offsets || !out) return 11;
+  rt_clear_error();
+  if (!enqueue_kq_rows(b, reinterpret_cast<__half const*>(x), out, offsets, n, bpr, experts, total_rows, qtype, rt_device_status_ptr(),
+                       static_cast<cudaStream_t>(stream))) return 40;
+  return rt_check_launch("raw-block MoE GEMV enqueue") ? 0 : kRuntimeError;
+}
+
 extern "C" int quactlize_ppu_dequantize(uint8_t const* b, int64_t block_bytes, uint16_t* out, int count, int qtype) {
   if (kq::raw_bytes(qtype) == 0) return 3;
   if (block_bytes != kq::raw_bytes(qtype) || count <= 0 || !b || !out) return 12;

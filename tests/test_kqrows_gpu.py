@@ -60,3 +60,17 @@ def test_blocks_off_a_16_byte_boundary(qt):
         view.copy_(_cuda(blocks))
         out = qb.gguf_vecdot_rows(view, _cuda(x), n, k, qt).cpu().numpy()
         assert kq.max_rel(out, want) < 2e-5, shift
+
+
+def test_moe_refuses_bad_offsets():
+    """Offsets that do not describe the rows raise, whatever was enqueued meanwhile, and the next call is right."""
+    e, n, k = 3, 64, 1024
+    blocks = synth.kquant_blocks(12, e * n * k // 256, seed=5).reshape(e, n * k // 256, -1)
+    x = synth.activations(6, k, seed=3)
+    b, xx = _cuda(blocks), _cuda(x)
+    for bad in ([0, 2, 4, 5], [1, 2, 4, 6], [0, 5, 2, 6], [0, -3, 4, 6], [0, 2, 400000, 6], [0, 2, 6]):
+        with pytest.raises(RuntimeError):
+            qb.gguf_vecdot_moe(b, xx, torch.tensor(bad, dtype=torch.int32, device=DEV), 12)
+    off = np.array([0, 0, 5, 6], dtype=np.int32)
+    out = qb.gguf_vecdot_moe(b, xx, _cuda(off), 12).cpu().numpy()
+    assert kq.max_rel(out, kq.vecdot_moe(blocks, x, off, n, k, 12)) < 2e-5

@@ -39,6 +39,7 @@ def _calls(qtype, n, m):
         "dequantize": lambda: qb.gguf_dequantize(b, qtype),
         "bc": lambda: qb.gguf_gemv_bc(one, low, high, units, qtype),
         "scale_first": lambda: qb.gguf_gemv_scale_first(x, *sf, qtype),
+        "moe": lambda: qb.gguf_vecdot_moe(b.view(2, -1, b.shape[1]), x, off, qtype),
         "plane": lambda: qb.gemv_plane(x, lo[:1], None, sc[:1], ze[:1], 4, 0, 64),
         "plane_no_zero": lambda: qb.gemv_plane(x, lo[:1], None, sc[:1], None, 4, 0, 64, code_offset=-8),
         "plane_two": lambda: qb.gemv_plane(x, sf[0], sf[1] if g.hi_bits else None, sf[2], sf[3], g.lo_bits, g.hi_bits, g.group_size),
