@@ -32,6 +32,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -60,6 +62,7 @@ struct GemmArgs {
   int code_offset, has_zero;
   int splits;              // K slices (gridDim.z); > 1: slice z accumulates its own 128-k pieces and writes fp32 to `partial`
   float* partial;          // [splits][m_rows][n] fp32 (split-K only), summed by splitk_reduce_kernel
+  int cluster;             // 1: the slices of a tile are one cluster, which adds them through shared memory; no `partial`
   unsigned long long const* out_rows;   // optional: the address output row r is stored at (n elements), instead of out + r*n
   unsigned int* status;
 };
@@ -352,8 +355,12 @@ mixed_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   constexpr int kDqWarps = 4 * MT * DQ;                       // the first 4*MT of them also run the epilogue: one per 32 accumulator lanes
   constexpr int NC = 8 * NTB / MT / DQ;                       // 8-element chunks a dequant thread converts per stage
   static_assert(NC >= 1 && NC * MT * DQ == 8 * NTB, "the dequant threads tile a stage's chunks exactly");
+  constexpr bool kCanCluster = MT == 1 && NT == 1;
+  constexpr int kSumPitch = kTN + 4;                          // floats between the rows of a slice's sums (off the bank period)
+  static_assert(!kCanCluster || offsetof(SM, a_full) >= size_t(kTM) * kSumPitch * 4, "the sums lie below the barriers");
   uint32_t const crank = PAIR ? cluster_ctarank() : 0u;
   SM& sm = *reinterpret_cast<SM*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  float* const smem_sums = reinterpret_cast<float*>(&sm);
   int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // ---- which tile: blockIdx.x = weight-column tile, blockIdx.y = row tile (grouped: searched in the per-expert counts)
@@ -568,7 +575,15 @@ mixed_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
             : "r"(taddr) : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (S > 1) {                                           // fp32 partial sums of this K slice
+        if (kCanCluster && g.cluster) {                        // this slice's sums, for the cluster to add: over the drained rings
+          if (row < mrows) {
+            float4* dst = reinterpret_cast<float4*>(smem_sums + row * kSumPitch + c);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              dst[u] = make_float4(__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1]), __uint_as_float(v[4 * u + 2]),
+                                   __uint_as_float(v[4 * u + 3]));
+          }
+        } else if (S > 1) {                                    // fp32 partial sums of this K slice
           if (row < mrows) {
             float4* dst = reinterpret_cast<float4*>(g.partial + (size_t(z) * g.m_rows + size_t(m0 + row)) * g.n + n0 + c);
 #pragma unroll
@@ -603,6 +618,33 @@ mixed_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     for (int s = 0; s < RST; ++s) { (void)mbar_wait_bounded(&sm.raw_full[s], 0, nullptr, 0, 100000000ull); (void)mbar_wait_bounded(&sm.raw_full[s], 1, nullptr, 0, 100000000ull); }
   }
   __syncthreads();
+  if constexpr (kCanCluster) {
+    if (g.cluster) {
+      // every slice's sums are in its CTA's shared memory: each CTA adds a run of the rows, in slice order
+      cluster_sync_all();
+      int const r0 = mrows * z / S, r1 = mrows * (z + 1) / S;
+      for (int i = threadIdx.x; i < (r1 - r0) * (kTN / 4); i += blockDim.x) {
+        int const row = r0 + i / (kTN / 4), c = i % (kTN / 4) * 4;
+        uint32_t const at = smem_u32(smem_sums + row * kSumPitch + c);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int w = 0; w < S; ++w) {
+          float4 o;
+          asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(cluster_addr(at, w)) : "memory");
+          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+        }
+        uint2 pk;
+        if constexpr (BF16) {
+          __nv_bfloat162 const h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
+          pk = make_uint2(*reinterpret_cast<uint32_t const*>(&h0), *reinterpret_cast<uint32_t const*>(&h1));
+        } else {
+          __half2 const h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+          pk = make_uint2(*reinterpret_cast<uint32_t const*>(&h0), *reinterpret_cast<uint32_t const*>(&h1));
+        }
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(g.out) + size_t(m0 + row) * g.n + n0 + c) = pk;
+      }
+      cluster_sync_all();                                     // nobody's sums go while another CTA may read them
+    }
+  }
   if constexpr (PAIR) cluster_sync_all();                     // neither CTA's shared or tensor memory goes while the other may use it
   if (warp == 2) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1039,8 +1081,9 @@ int launch_mixed_gemm(GemmDesc const& d, cudaStream_t stream) {
   g.out = d.out; g.m_rows = d.total_rows; g.n = d.n; g.k = d.k; g.experts = E; g.group_size = gs;
   g.code_offset = d.code_offset; g.has_zero = d.zero ? 1 : 0;
   int const splits = d.splits > 1 ? d.splits : 1;
-  if (splits > d.k / kRawK || splits > 64 || (splits > 1 && !d.partial)) return 30;    // every slice owns at least one piece
-  g.splits = splits; g.partial = d.partial;
+  bool const cluster = MT == 1 && NT == 1 && splits > 1 && d.cluster;
+  if (splits > d.k / kRawK || splits > 64 || (splits > 1 && !d.partial && !cluster) || (cluster && splits > 8)) return 30;    // every slice owns at least one piece
+  g.splits = splits; g.partial = d.partial; g.cluster = cluster ? 1 : 0;
   g.out_rows = d.out_rows;
   if (d.out_rows && splits > 1) return 30;                     // the reduce kernel writes the dense layout only
   g.status = rt_device_status_ptr();
@@ -1088,6 +1131,18 @@ int launch_mixed_gemm(GemmDesc const& d, cudaStream_t stream) {
       (void)cudaGetLastError();
       return kRuntimeError;
     }
+    return 0;
+  }
+  if (cluster) {                                               // the K slices of a tile are neighbours along grid z
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(d.n / kTN, mtiles, splits);
+    cfg.blockDim = dim3(128 + 128 * MT * gemm_dq<MT, NT, DEPTH>());
+    cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = unsigned(splits);
+    cfg.attrs = at; cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, ma, ml, mh, ms, mz, g) != cudaSuccess) { (void)cudaGetLastError(); return kRuntimeError; }
     return 0;
   }
   kern<<<dim3((d.n + kTN * NT - 1) / (kTN * NT), mtiles, splits), 128 + 128 * MT * gemm_dq<MT, NT, DEPTH>(), smem, stream>>>(ma, ml, mh, ms, mz, g);
@@ -1154,16 +1209,53 @@ bool tma_make_map(CUtensorMap* m, CUtensorMapDataType dt, int rank, void const* 
 
 long long gemm_swap_launches() { return g_swap_launches.load(std::memory_order_relaxed); }
 
-int enqueue_mixed_gemm(GemmDesc const& d, cudaStream_t stream) {
+// Which form a problem takes: the 256 x 256 tile (one CTA per SM), or 128 x 128 tiles on two-deep rings (two CTAs per SM), for a
+// dense problem with K cut over a cluster of 2, 4 or 8 CTAs that add their slices through shared memory.  Microseconds, from
+// 64-k stages: a wave of 256 x 256 tiles 6 + 0.9 a stage whatever its rows; of 128 x 128 tiles 0.6 a stage with one CTA on an
+// SM and 0.78 with two, and 5 for the pipeline's fill, drain and launch (7 with the exchange of a cluster, 8 with eight CTAs).
+// Measured on 4096-deep int4, us: m = 17, n = 1024 37.7 -> 12.7 (8 slices); m = 256, n = 4096 59.9 -> 23.0 (4); m = 190,
+// n = 14336 77 -> 54.6 (none); m = 333, n = 14336 62.6 as 256 x 256 tiles, 85-95 as the others.  Ragged problems are not cut
+// in K: a row's bits then do not depend on which other rows, experts or ranks share the launch.  Nor are dense ones of up to
+// 2048 k, where the cut gives least (m = 190, n = k = 1024: 10.7 against 14.7): there every form of the kernel, and an expert
+// alone against its rows of a ragged launch, agree to the last bit.  The tile counts of ragged problems are an estimate (half
+// a tile is padding per expert): 8 experts, 1200 rows, n = 8192 225 -> 118.
+struct GemmForm { bool big; int splits; };
+GemmForm gemm_form(GemmDesc const& d) {
+  double const stages = d.k / kTK;
+  int const sms = rt_sm_count();
+  auto row_tiles = [&](int t) {
+    return d.experts > 0 ? double(d.total_rows) / t + 0.5 * std::min(d.experts, d.total_rows) : double((d.total_rows + t - 1) / t);
+  };
+  double const tiles256 = std::ceil(row_tiles(256) * ((d.n + 255) / 256)), tiles128 = std::ceil(row_tiles(128) * (d.n / kTN));
+  GemmForm best{true, 1};
+  double best_us = std::ceil(tiles256 / sms) * (6.0 + 0.9 * stages);
+  for (int S : {1, 2, 4, 8}) {
+    if (S > 1 && (d.experts > 0 || d.out_rows || d.k <= 2048)) break;
+    double const ctas = tiles128 * S, full = std::floor(ctas / (2 * sms)), rest = ctas - full * 2 * sms;
+    double const fixed = S == 1 ? 5.0 : S < 8 ? 7.0 : 8.0, per = stages / S;
+    double const us = full * (fixed + 0.78 * per) + (rest > 0 ? fixed + (rest > sms ? 0.78 : 0.6) * per : 0.0);
+    if (us < best_us) { best_us = us; best = GemmForm{false, S}; }
+  }
+  return best;
+}
+
+int enqueue_mixed_gemm(GemmDesc const& given, cudaStream_t stream) {
+  GemmDesc d = given;
   if (!d.act || !d.low || !d.scale || (!d.out && !d.out_rows) || d.total_rows <= 0 || d.n <= 0 || d.n % kTN || d.k <= 0 || d.k % 256 ||
       d.group_size < 16 || (d.group_size & (d.group_size - 1)) || d.k % d.group_size || (d.hi_bits && !d.high) ||
       (d.experts > 0 && !d.offsets)) return 30;
   auto al = [](void const* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (!al(d.act) || !al(d.low) || !al(d.scale) || (d.out && !al(d.out)) || (d.zero && !al(d.zero)) || (d.hi_bits && !al(d.high))) return 30;
   int const key = d.lo_bits * 10 + d.hi_bits;
-  // 256 x 256 CTA tiles (four accumulators = all 512 TMEM columns) for prefill-sized problems; small ones keep 128 x 128
   int const avg_rows = d.experts > 0 ? d.total_rows / d.experts : d.total_rows;
-  bool const big = d.tile == 256 || d.tile == 512 || d.tile == 1024 || (d.tile == 0 && avg_rows >= 192);
+  bool big = d.tile == 256 || d.tile == 512 || d.tile == 1024 || (d.tile == 0 && avg_rows >= 192);
+  char const* const swap_env = std::getenv("QUACTLIZE_B200_GEMM_SWAP");   // set: prefill-sized problems; "all": every size
+  bool const pair_on = std::getenv("QUACTLIZE_B200_GEMM_PAIR") != nullptr;
+  if (d.tile == 0 && d.splits <= 1 && !d.shallow && !swap_env && !pair_on) {
+    GemmForm const f = gemm_form(d);
+    big = f.big;
+    if (!big) { d.shallow = 1; d.splits = f.splits; d.cluster = f.splits > 1 ? 1 : 0; }
+  }
   if (d.shallow && !big) {                        // decode tactic: 128 x 128 tiles, two-deep rings, several CTAs per SM
 #define QB_GEMM_SHALLOW(K, L, H) case K: return d.act_bf16 ? launch_mixed_gemm<L, H, true, 1, 1, 1>(d, stream) : launch_mixed_gemm<L, H, false, 1, 1, 1>(d, stream);
     switch (key) {
@@ -1181,11 +1273,9 @@ int enqueue_mixed_gemm(GemmDesc const& d, cudaStream_t stream) {
   // The swapped form (weights as the A operand, converted into tensor memory): int4 planes, whole 256-row weight tiles,
   // one K slice.  Opt-in (QUACTLIZE_B200_GEMM_SWAP in the environment, read per call, or tile = 1024): it is slower than
   // the tiles below on the problems measured (see mixed_gemm_swap_kernel).
-  char const* const swap_env = std::getenv("QUACTLIZE_B200_GEMM_SWAP");   // set: prefill-sized problems; "all": every size
   bool const swap_on = swap_env != nullptr && (big || swap_env[0] == 'a');
   if (key == 40 && d.splits <= 1 && !d.shallow && d.n % (2 * kTN) == 0 && (d.tile == 1024 || (d.tile == 0 && swap_on)))
     return d.act_bf16 ? launch_mixed_gemm_swap<true>(d, stream) : launch_mixed_gemm_swap<false>(d, stream);
-  bool const pair_on = std::getenv("QUACTLIZE_B200_GEMM_PAIR") != nullptr;
   if (big && key == 40 && d.n % 256 == 0 && d.splits <= 1 && (d.tile == 512 || (d.tile == 0 && pair_on)))
     return d.act_bf16 ? launch_mixed_gemm<4, 0, true, 2, 2, 2>(d, stream) : launch_mixed_gemm<4, 0, false, 2, 2, 2>(d, stream);
 #define QB_GEMM_CASE(K, L, H) case K: return d.act_bf16 ? (big ? launch_mixed_gemm<L, H, true, 2, 2>(d, stream) : launch_mixed_gemm<L, H, true, 1, 1>(d, stream)) \

@@ -65,6 +65,7 @@ struct GemmDesc {
   int tile;                   // 0 = chosen from the problem size, 128 / 256 = that CTA tile (the two compiled tactics)
   int splits;                 // split-K slices; 0 or 1 = none.  > 1 needs `partial` and at most k/128 slices
   float* partial;             // fp32 [splits][total_rows][n] workspace of the split-K form (caller-owned)
+  int cluster;                // with splits 2..8 and 128 x 128 tiles: the slices add up inside a cluster, no `partial`
   int shallow;                // 1 = the decode tactic: 128 x 128 tiles with two-deep rings (several CTAs per SM)
   unsigned long long const* out_rows;   // optional device array [total_rows]: where each output row goes (see GemmArgs)
 };

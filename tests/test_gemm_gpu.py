@@ -241,3 +241,29 @@ def test_swapped_form_is_bit_identical(case, monkeypatch):
     torch.cuda.synchronize()
     assert torch.equal(got, ref)
     assert L.quactlize_b200_device_wait_status() == 0
+
+
+# K cut over a cluster (dense, more than 2048 k): slices of unequal length (k / 128 not a multiple of the cluster), row tiles
+# that end early, one column tile and several, every plane width, results against the oracle as for the whole-K form
+@pytest.mark.parametrize("m,n,k", [(1, 128, 2304), (17, 128, 8192), (129, 256, 2560), (130, 1024, 4096), (190, 384, 4352), (300, 2048, 2304)])
+@pytest.mark.parametrize("bits,gs,zero,dtype", [(4, 32, True, torch.float16), (4, 128, False, torch.bfloat16), (2, 64, True, torch.bfloat16)])
+def test_k_cut_over_a_cluster(m, n, k, bits, gs, zero, dtype):
+    low, scale, zp = synth.group_planes(1, n, k, bits, gs, seed=m + n)
+    a = torch.from_numpy(synth.activations(m, k, seed=m, dtype=np.float32)).to(dtype)
+    shift = 0 if zero else -(1 << (bits - 1))
+    call = lambda: qb.gemm_plane(a.to(DEV), _cuda(low), None, _cuda(scale), _cuda(zp) if zero else None, bits, 0, gs, code_offset=shift)
+    out = call()
+    want = kq.planes_matmul(a.float().numpy(), low, None, scale, zp, bits, 0, gs)
+    _check(out, want, dtype == torch.bfloat16)
+    assert torch.equal(out, call())                                      # slices are added in a fixed order
+    assert _lib.lib().quactlize_b200_device_wait_status() == 0
+
+
+@pytest.mark.parametrize("qt", [11, 13, 14])
+def test_k_cut_over_a_cluster_two_planes(qt):
+    m, n, k = 70, 256, 3072
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=qt)
+    low, high, units = (t.to(DEV) for t in qb.gguf_prepare_fully_quantized_dense(torch.from_numpy(blocks), n, k, qt))
+    a = synth.activations(m, k, seed=4)
+    out = qb.gguf_dense_fully_quantized(_cuda(a), low, high, units, qt)
+    _check(out, a.astype(np.float64) @ kq.dequantize_f32(blocks, qt).reshape(n, k).T.astype(np.float64))
