@@ -323,7 +323,7 @@ def run_b200(args):
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm"], "unit": "GB/s",
                      "frac": round(achieved / peaks["hbm"], 4), "frac_of_nominal_8000": round(achieved / 8000.0, 4),
                      "traffic": traffic, "traffic_source": traffic_src,
-                     "peak_source": peaks["source"], "kernel": "q4k_gemv1_kernel" if m == 1 else "q4k_rows_kernel",
+                     "peak_source": peaks["source"], "kernel": "q4k_gemv1_kernel" if m == 1 else "kq_rows_kernel",
                      "algorithmic_bytes_per_launch": alg, "us_per_launch": round(per_launch_ms * 1e3, 3)},
         "e2e": {"value": round(e2e_val, 3), "unit": "GB/s", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                 "api": "quactlize_ppu_vecdot_dense (host pointers, pinned)", "steps": e2e_steps},

@@ -24,6 +24,10 @@
 //
 // Rows of 84-, 110- and 210-byte blocks are read in 4-byte words, the word order rotated by the lane's quarter: rows lie
 // 16 bytes off a 128-byte pitch, so the 32 lanes of a load fall on 32 banks.  Every wait is bounded.
+//
+// Measured, 4096 -> 14336, eight rows, us: Q4_K 15.5 -> 13.4 (33 MB, 2.5 TB/s), Q2_K 41 -> 14.8, Q3_K 64 -> 16.6, Q5_K 58 -> 15.9,
+// Q6_K 66 -> 19.6.  What bounds it is the latency of a tile round, 1.13 us for Q4_K against 0.83 us of stream: about 260
+// instructions a warp, half of them on the half-rate integer pipe, with four to five warps per scheduler.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 

@@ -108,7 +108,7 @@ def cfg2(m: int, n: int, k: int, dev="cuda:0", qtype: int = 12) -> Case:
         return {"kind": "raw", "got": got, "blocks": sub, "x": x, "n": len(cols), "k": k, "qtype": qtype, "out": "fp32"}
     wb = blocks.size
     name = {10: "q2k", 11: "q3k", 12: "q4k", 13: "q5k", 14: "q6k"}.get(qtype, f"qt{qtype}")
-    kernel = "kquant_gemv_generic_kernel" if qtype != 12 else "q4k_gemv1_kernel" if m == 1 else "q4k_rows_kernel"
+    kernel = ("q4k_gemv1_kernel" if qtype == 12 else "kquant_gemv1_kernel") if m == 1 else "kq_rows_kernel"
     return Case(f"cfg2_{name}_m{m}_{k}to{n}", "hbm", wb, wb + m * k * 2 + m * n * 4, 2.0 * m * n * k, nc, launch, sample, kernel)
 
 
