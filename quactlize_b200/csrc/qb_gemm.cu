@@ -1209,8 +1209,9 @@ bool tma_make_map(CUtensorMap* m, CUtensorMapDataType dt, int rank, void const* 
 
 long long gemm_swap_launches() { return g_swap_launches.load(std::memory_order_relaxed); }
 
-// Which form a problem takes: the 256 x 256 tile (one CTA per SM), or 128 x 128 tiles on two-deep rings (two CTAs per SM), for a
-// dense problem with K cut over a cluster of 2, 4 or 8 CTAs that add their slices through shared memory.  Microseconds, from
+// Which form a problem takes: the 256 x 256 tile (one CTA per SM), or 128 x 128 tiles, on four-deep rings where an SM gets one
+// CTA (m = 17, n = 4096 39.3 against 41.6 us) and on two-deep ones, two CTAs per SM, where there are more; for a dense problem
+// with K cut over a cluster of 2, 4 or 8 CTAs that add their slices through shared memory.  Microseconds, from
 // 64-k stages: a wave of 256 x 256 tiles 6 + 0.9 a stage whatever its rows; of 128 x 128 tiles 0.6 a stage with one CTA on an
 // SM and 0.78 with two, and 5 for the pipeline's fill, drain and launch (7 with the exchange of a cluster, 8 with eight CTAs).
 // Measured on 4096-deep int4, us: m = 17, n = 1024 37.7 -> 12.7 (8 slices); m = 256, n = 4096 59.9 -> 23.0 (4); m = 190,
@@ -1218,23 +1219,25 @@ long long gemm_swap_launches() { return g_swap_launches.load(std::memory_order_r
 // in K: a row's bits then do not depend on which other rows, experts or ranks share the launch.  Nor are dense ones of up to
 // 2048 k, where the cut gives least (m = 190, n = k = 1024: 10.7 against 14.7): there every form of the kernel, and an expert
 // alone against its rows of a ragged launch, agree to the last bit.  The tile counts of ragged problems are an estimate (half
-// a tile is padding per expert): 8 experts, 1200 rows, n = 8192 225 -> 118.
-struct GemmForm { bool big; int splits; };
+// a tile is padding per expert, one tile at least): 8 experts, 1200 rows, n = 8192 225 -> 118.
+struct GemmForm { bool big, shallow; int splits; };
 GemmForm gemm_form(GemmDesc const& d) {
   double const stages = d.k / kTK;
   int const sms = rt_sm_count();
   auto row_tiles = [&](int t) {
-    return d.experts > 0 ? double(d.total_rows) / t + 0.5 * std::min(d.experts, d.total_rows) : double((d.total_rows + t - 1) / t);
+    if (d.experts <= 0) return double((d.total_rows + t - 1) / t);
+    double const held = std::min(d.experts, d.total_rows);
+    return std::max(held, double(d.total_rows) / t + 0.5 * held);
   };
   double const tiles256 = std::ceil(row_tiles(256) * ((d.n + 255) / 256)), tiles128 = std::ceil(row_tiles(128) * (d.n / kTN));
-  GemmForm best{true, 1};
+  GemmForm best{true, false, 1};
   double best_us = std::ceil(tiles256 / sms) * (6.0 + 0.9 * stages);
   for (int S : {1, 2, 4, 8}) {
     if (S > 1 && (d.experts > 0 || d.out_rows || d.k <= 2048)) break;
     double const ctas = tiles128 * S, full = std::floor(ctas / (2 * sms)), rest = ctas - full * 2 * sms;
     double const fixed = S == 1 ? 5.0 : S < 8 ? 7.0 : 8.0, per = stages / S;
     double const us = full * (fixed + 0.78 * per) + (rest > 0 ? fixed + (rest > sms ? 0.78 : 0.6) * per : 0.0);
-    if (us < best_us) { best_us = us; best = GemmForm{false, S}; }
+    if (us < best_us) { best_us = us; best = GemmForm{false, S > 1 || ctas > sms, S}; }
   }
   return best;
 }
@@ -1254,7 +1257,7 @@ int enqueue_mixed_gemm(GemmDesc const& given, cudaStream_t stream) {
   if (d.tile == 0 && d.splits <= 1 && !d.shallow && !swap_env && !pair_on) {
     GemmForm const f = gemm_form(d);
     big = f.big;
-    if (!big) { d.shallow = 1; d.splits = f.splits; d.cluster = f.splits > 1 ? 1 : 0; }
+    if (!big) { d.shallow = f.shallow ? 1 : 0; d.splits = f.splits; d.cluster = f.splits > 1 ? 1 : 0; }
   }
   if (d.shallow && !big) {                        // decode tactic: 128 x 128 tiles, two-deep rings, several CTAs per SM
 #define QB_GEMM_SHALLOW(K, L, H) case K: return d.act_bf16 ? launch_mixed_gemm<L, H, true, 1, 1, 1>(d, stream) : launch_mixed_gemm<L, H, false, 1, 1, 1>(d, stream);
