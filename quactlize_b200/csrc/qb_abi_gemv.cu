@@ -150,8 +150,9 @@ extern "C" int quactlize_b200_vecdot_moe_dev_v1(uint8_t const* b, int64_t block_
   return rt_check_launch("raw-block MoE GEMV enqueue") ? 0 : kRuntimeError;
 }
 
-// The same launch through the one kernel that clamps the offsets to [0, total_rows] and their differences to >= 0: it stays in
-// bounds whatever they hold, so a caller may enqueue it before the offsets are checked.  40: a form it does not cover.
+// The same launch through the one kernel that settles the offsets itself (clamped to [0, total_rows], none below the one before):
+// it stays in bounds and does no more work than total_rows rows make, whatever they hold, so a caller may enqueue it before
+// they are checked.  40: a form it does not cover.
 extern "C" int quactlize_b200_vecdot_moe_clamped_dev_v1(uint8_t const* b, int64_t block_bytes, uint16_t const* x, int const* offsets,
                                                         float* out, int n, int bpr, int experts, int total_rows, int qtype, void* stream) {
   if (kq::raw_bytes(qtype) == 0) return 2;

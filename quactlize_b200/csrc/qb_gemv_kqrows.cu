@@ -39,6 +39,7 @@
 
 #include "qb_device.cuh"
 #include "qb_internal.hpp"
+#include "qb_kqrows_units.hpp"
 #include "qb_kquant.cuh"
 #include "qb_runtime.hpp"
 
@@ -47,7 +48,7 @@ namespace {
 
 constexpr int kKrWarps = 16;                       // computing warps
 constexpr int kKrThreads = (kKrWarps + 2) * 32;
-constexpr int kKrTile = 16, kKrCols = 8;
+constexpr int kKrTile = 16;
 constexpr int kKrMaxStages = 8;
 constexpr int kKrMaxExperts = 1024;
 constexpr int kKrAccTiles = 16;                    // tiles whose sums the reducing warp carries over K passes and CTAs
@@ -458,15 +459,27 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
   }
   // Under programmatic dependent launch nothing of the activations, the offsets or the output is touched before this.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  int groups = (a.m_rows + kKrCols - 1) / kKrCols;
+  int groups = kr_groups(a.m_rows);
   if (a.offsets) {
-    for (int i = threadIdx.x; i <= a.experts; i += kKrThreads) off[i] = min(max(a.offsets[i], 0), a.m_rows);
+    // The offsets may not have been checked: they are settled first, so that no later index depends on what else they hold.
+    for (int i = threadIdx.x; i <= a.experts; i += kKrThreads) off[i] = a.offsets[i];
     __syncthreads();
-    if (warp == 0) {                                                // inclusive scan of the experts' group counts
-      int carry = 0;
+    if (warp == 0) {
+      int top = 0;
+      for (int base = 0; base <= a.experts; base += 32) {           // running maximum of the clamped offsets
+        int const i = base + lane;
+        int v = kr_settle(0, i <= a.experts ? off[i] : 0, a.m_rows);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { int const p = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v = kr_settle(p, v, a.m_rows); }
+        v = kr_settle(top, v, a.m_rows);
+        if (i <= a.experts) off[i] = v;
+        top = __shfl_sync(0xffffffffu, v, 31);
+      }
+      __syncwarp();
+      int carry = 0;                                                // inclusive scan of the experts' group counts
       for (int base = 0; base < a.experts; base += 32) {
         int const i = base + lane;
-        int v = i < a.experts ? (max(off[i + 1] - off[i], 0) + kKrCols - 1) / kKrCols : 0;
+        int v = i < a.experts ? kr_groups(off[i + 1] - off[i]) : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { int const p = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += p; }
         v += carry;
@@ -481,8 +494,8 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
   long long const units = (long long)groups * a.tiles;
   unsigned const part_i = blockIdx.x / a.C, part_n = gridDim.x / a.C;
   KrWalk wk{};
-  wk.u = int(units * part_i / part_n);
-  wk.u_end = int(units * (part_i + 1) / part_n);
+  wk.u = kr_cut(units, part_i, part_n);
+  wk.u_end = kr_cut(units, part_i + 1, part_n);
   int const* offp = a.offsets ? off : nullptr;
   bool dead = false;
 
@@ -691,8 +704,8 @@ template <int QT>
 bool launch(KrArgs a, cudaStream_t stream) {
   a.tiles = (a.n + kKrTile - 1) / kKrTile;
   a.xrows = std::min(kKrCols, a.m_rows);
-  int const most = a.offsets ? std::min(a.m_rows, a.m_rows / kKrCols + a.experts) : (a.m_rows + kKrCols - 1) / kKrCols;   // groups
-  if ((long long)most * a.tiles > (1ll << 29)) return false;
+  int const most = a.offsets ? kr_most_groups(a.m_rows, a.experts) : kr_groups(a.m_rows);
+  if ((long long)most * a.tiles > kKrMaxUnits) return false;
   // a router that spreads r rows over E experts touches about r of them while r is small against E
   int const likely = a.offsets ? std::max(1, std::min(most, int((long long)a.m_rows * a.experts / (a.m_rows + a.experts)))) : most;
   KrPlan const p = kr_plan<QT>(a.bpr, likely * a.tiles, a.xrows, a.experts);

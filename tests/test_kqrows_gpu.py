@@ -10,7 +10,7 @@ import torch
 
 import quactlize_b200 as qb
 from oracle import kquant as kq
-from quactlize_b200 import synth
+from quactlize_b200 import _lib, synth
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -74,3 +74,22 @@ def test_moe_refuses_bad_offsets():
     off = np.array([0, 0, 5, 6], dtype=np.int32)
     out = qb.gguf_vecdot_moe(b, xx, _cuda(off), 12).cpu().numpy()
     assert kq.max_rel(out, kq.vecdot_moe(blocks, x, off, n, k, 12)) < 2e-5
+
+
+@pytest.mark.parametrize("off,used", [([0, 6, 0, 6, 0], [6, 0, 0, 0]), ([2, 1, 5, 3, 9], [0, 3, 0, 1]), ([-4, 6, -1, 2, 7], [6, 0, 0, 0])])
+def test_unchecked_offsets_are_settled(off, used):
+    """The entry that may be enqueued before its offsets are checked: offsets are clamped to the rows and never fall, so a row
+    belongs to one expert and the rows of the others are left alone."""
+    e, n, k, rows = 4, 40, 768, 6
+    blocks = synth.kquant_blocks(12, e * n * k // 256, seed=8).reshape(e, n * k // 256, -1)
+    x = synth.activations(rows, k, seed=4)
+    b, xx, out = _cuda(blocks), _cuda(x), torch.full((rows, n), 77.0, device=DEV)
+    o = torch.tensor(off, dtype=torch.int32, device=DEV)
+    rc = _lib.lib().quactlize_b200_vecdot_moe_clamped_dev_v1(b.data_ptr(), b.shape[2], xx.data_ptr(), o.data_ptr(), out.data_ptr(), n, k // 256,
+                                                             e, rows, 12, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    first = min(max(off[0], 0), rows)
+    settled = np.concatenate([[0], np.cumsum(used)]).astype(np.int32)
+    want = np.full((rows, n), 77.0, dtype=np.float32)
+    want[first:first + settled[-1]] = kq.vecdot_moe(blocks, x[first:first + settled[-1]], settled, n, k, 12)
+    assert kq.max_rel(out.cpu().numpy(), want) < 2e-5
