@@ -320,7 +320,9 @@ __global__ void __launch_bounds__(kQ4Warps * 32, 1) q4k_gemv1_kernel(Q4Args a) {
   }
 
   // ---- 6. main loop: one stage = the segments of two consecutive rows -------------------------------------------------
-  uint32_t const lane_off = uint32_t(blk) * 144u;
+  // Lanes without a block read block 0.  At their own place (up to 2304 bytes into a segment of nbs * 144) the last warp's
+  // second stage would be read past the ring and, with few rows per CTA, past the shared memory: K < 4096, over 62 rows a CTA.
+  uint32_t const lane_off = uint32_t(active ? blk : 0) * 144u;
   uint32_t const code_off = lane_off + 16u + uint32_t(prt) * 64u;
   uint32_t const mask_a = prt ? 0x0F0F0F0Fu : 0x3F3F3F3Fu, mask_b = prt ? 0x30303030u : 0u;
   uint32_t st_addr = ring32, st_bar = bar32;

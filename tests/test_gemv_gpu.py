@@ -113,6 +113,17 @@ def test_q4k_fast_kernel_vs_oracle(n, k, m):
     _wait_ok()
 
 
+# Rows of fewer than 16 blocks with every ring stage of a CTA in use (more than 62 rows per CTA): the lanes without a block
+# must stay inside the CTA's shared memory, in the last warp's last stage too.
+@pytest.mark.parametrize("n,k", [(14336, 2048), (9400, 3072), (16384, 1024), (9300, 256)])
+def test_q4k_short_rows_fill_every_stage(n, k):
+    blocks = synth.kquant_blocks(12, n * k // 256, seed=k)
+    x = synth.activations(1, k, seed=n)
+    out = qb.gguf_vecdot_dense(_cuda(blocks), _cuda(x), n, k, 12).cpu().numpy()
+    assert kq.max_rel(out, kq.vecdot_dense(blocks, x, n, k, 12)) < 4e-3
+    assert _lib.lib().quactlize_b200_device_wait_status() == 0
+
+
 KQ_SHAPES = [(256, 4096), (96, 14336), (37, 2048), (1, 4096), (130, 8192), (300, 6144)]
 
 
