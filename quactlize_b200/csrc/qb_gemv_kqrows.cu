@@ -17,7 +17,7 @@
 // Structure.  One CTA per SM: 16 computing warps, a copy warp, a reducing warp.  K is covered in passes of P superblocks,
 // and for deep rows cut over the CTAs of a cluster; warp (slot, b) owns superblock b of the pass and keeps its B fragments
 // in registers over all tiles; a ring stage is RS tiles of 16 rows x P superblocks, one cp.async.bulk per row (rows off a
-// 16-byte boundary are copied from the boundary below).  The activations of a pass arrive through shared memory the same
+// 16-byte boundary are copied from the boundary below, and nothing outside the tensor is read).  The activations of a pass arrive through shared memory the same
 // way, a pass ahead (the very first ones by plain loads).  The K slices of a tile are added in warp order, then in CTA order, by the reducing warp (results do
 // not depend on timing) while the others work on the next tile.  The tiles of all (expert, eight-row group) pairs form one
 // list that is cut evenly over the clusters: empty experts cost nothing and a launch is one wave whatever the router does.
@@ -502,6 +502,7 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
   if (warp == kKrWarps) {
     // ---- copies ---------------------------------------------------------------------------------------------------------
     KrRing ws{}, xr{};
+    uintptr_t const lo = reinterpret_cast<uintptr_t>(a.blocks), hi = lo + size_t(a.offsets ? a.experts : 1) * a.n * a.bpr * kBytes;
     bool first = a.xrows <= kKrDirectRows;                          // the computing warps load these activations themselves
     while (!dead && wk.next(a, offp, cum)) {
       for (int p = 0; p < a.passes && !dead; ++p) {
@@ -521,20 +522,29 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
         for (int tb = wk.t0; tb < wk.t1; tb += a.RS, ws.step(a.stages), src0 += size_t(a.RS * kKrTile) * step) {
           if (ws.lap && !mbar_wait_bounded(&bar->empty[ws.i], ws.phase ^ 1u, a.status, kWaitStageTimeout)) { dead = true; break; }
           int const rows = nb ? min(min(a.RS, wk.t1 - tb) * kKrTile, a.n - tb * kKrTile) : 0;
-          auto span = [&](int r, uint8_t const*& from) -> unsigned {    // the 16-byte units that hold row r's segment
-            uintptr_t const b = reinterpret_cast<uintptr_t>(src0 + size_t(r) * step);
-            from = reinterpret_cast<uint8_t const*>(b & ~uintptr_t(15));
-            return unsigned(((b + len + 15) & ~uintptr_t(15)) - (b & ~uintptr_t(15)));
-          };
+          uint8_t* const stage = ring + ws.i * stage_bytes;
+          auto span = [&](int r) { return kr_span(reinterpret_cast<uintptr_t>(src0 + size_t(r) * step), len, lo, hi); };
           unsigned total = 0;
-          uint8_t const* from;
-          for (int r = lane; r < rows; r += 32) total += span(r, from);
+          for (int r = lane; r < rows; r += 32) {
+            KrSpan const s = span(r);
+            total += unsigned(s.to - s.from);
+            if constexpr (QT != 12 && QT != 13) {                   // the ends of the tensor, off a 16-byte boundary
+              uintptr_t const b = reinterpret_cast<uintptr_t>(src0 + size_t(r) * step);
+              if (s.from > b || s.to < b + len) {
+                uint8_t* const dst = stage + size_t(r) * a.pitch;
+                for (uintptr_t p = b; p < s.from; ++p) dst[p - s.first] = __ldg(reinterpret_cast<uint8_t const*>(p));
+                for (uintptr_t p = s.to; p < b + len; ++p) dst[p - s.first] = __ldg(reinterpret_cast<uint8_t const*>(p));
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              }
+            }
+          }
           total = __reduce_add_sync(0xffffffffu, total);
+          __syncwarp();                                             // the bytes are written before lane 0 arrives
           if (lane == 0) mbar_expect_tx(&bar->full[ws.i], total);
           __syncwarp();
           for (int r = lane; r < rows; r += 32) {
-            unsigned const bytes = span(r, from);
-            bulk_g2s(ring + ws.i * stage_bytes + size_t(r) * a.pitch, from, bytes, &bar->full[ws.i]);
+            KrSpan const s = span(r);
+            bulk_g2s(stage + size_t(r) * a.pitch + (s.from - s.first), reinterpret_cast<void const*>(s.from), unsigned(s.to - s.from), &bar->full[ws.i]);
           }
         }
       }

@@ -46,3 +46,20 @@ def test_units_of_valid_offsets(units):
         counts = np.random.default_rng(seed).multinomial(rows, np.ones(experts) / experts)
         off = [0, *np.cumsum(counts).tolist()]
         assert units(rows, 7, 33, off)[0] == sum(-(-int(c) // 8) for c in counts)
+
+
+@pytest.fixture(scope="module")
+def spans(tmp_path_factory):
+    return _build(tmp_path_factory, "kqrows_span_probe")
+
+
+@pytest.mark.parametrize("block,align", [(84, 4), (110, 2), (210, 2), (144, 16), (176, 16)])
+def test_copies_stay_inside_the_tensor(spans, block, align):
+    """Bulk copies take whole 16-byte units; at the ends of a tensor that begins or ends off a boundary the rest is copied by the byte."""
+    for shift in range(0, 16, align):
+        for rows, bpr, sb in ((1, 1, 1), (3, 5, 5), (17, 9, 4), (2, 16, 16)):
+            text = f"{4096 + shift} {rows * bpr * block} {bpr * block} {sb * block}"
+            r = subprocess.run([spans], input=text, capture_output=True, text=True)
+            assert r.returncode == 0, (text, r.stdout)
+            aligned_ends = shift == 0 and (rows * bpr * block) % 16 == 0
+            assert (int(r.stdout) == 0) == aligned_ends, text
