@@ -50,7 +50,7 @@ constexpr int kKrWarps = 16;                       // computing warps
 constexpr int kKrThreads = (kKrWarps + 2) * 32;
 constexpr int kKrTile = 16;
 constexpr int kKrMaxStages = 8;
-constexpr int kKrMaxExperts = 1024;
+constexpr int kKrMaxExperts = 4096;                // their offsets and group counts: 32 KB of shared memory at most
 constexpr int kKrAccTiles = 16;                    // tiles whose sums the reducing warp carries over K passes and CTAs
 // The first activations of a CTA by plain loads of the computing warps: 0.3 us earlier than through shared memory at one to
 // four rows (Q4_K 2400 x 4096, 2 rows: 6.05 against 6.43 us), later at eight (14336 x 4096: 14.1 against 13.4 us).

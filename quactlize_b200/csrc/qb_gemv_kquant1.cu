@@ -45,8 +45,7 @@ struct KqArgs {
   uint8_t const* blocks;
   __half const* x;
   float* out;
-  int const* offsets;        // cumulative [experts+1] (grouped) or nullptr (dense)
-  int n, bpr, max_rows;      // grid.y = activation rows (dense) or experts*max_rows (grouped)
+  int n, bpr;                // grid.y = activation rows
   int S, nbs, RS;            // K segments per row, blocks per segment, row slots per CTA
   int seg_stride;            // bytes between the two row segments of a ring stage
   int rows_q, rows_r;        // n = gridDim.x*rows_q + rows_r: CTA c owns rows_q (+1 if c < rows_r) consecutive rows
@@ -266,18 +265,10 @@ __global__ void __launch_bounds__(kKqWarps * 32, 1) kquant_gemv1_kernel(KqArgs a
   extern __shared__ __align__(128) uint8_t smem[];
   int const T = blockDim.x, W = T >> 5, warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   int const seg = warp % a.S, rslot = warp / a.S;
-  int e = 0, arow;
-  // Under programmatic dependent launch the offsets and the activation may be the preceding kernel's output: nothing of
-  // them is read before this wait (it also precedes the early return of surplus CTAs).
+  int const arow = blockIdx.y;
+  // Under programmatic dependent launch the activation may be the preceding kernel's output: nothing of it is read before
+  // this wait.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (a.offsets) {
-    e = blockIdx.y / a.max_rows;
-    int const r = blockIdx.y % a.max_rows, r0 = a.offsets[e], r1 = a.offsets[e + 1];
-    if (r >= r1 - r0) return;                                     // uniform for the CTA
-    arow = r0 + r;
-  } else {
-    arow = blockIdx.y;
-  }
   int const bpr = a.bpr, k = bpr * 256;
   // shared memory map: activations (piece q of half-block slot s at (q*2*bpr + s)*16), group sums, scratch, rings, barriers
   uint32_t const s0 = smem_u32(smem);
@@ -316,7 +307,7 @@ __global__ void __launch_bounds__(kKqWarps * 32, 1) kquant_gemv1_kernel(KqArgs a
   // free stage (see qb_gemv_q4k.cu): the CTA's pairs rarely divide evenly over its warps.  Which warp computes a row does
   // not change the row's arithmetic.
   static_assert(kKqStages == 2, "the claim bookkeeping below keeps two pairs per warp");
-  uint8_t const* seg_base = a.blocks + (size_t(e) * a.n + size_t(row0)) * row_stride + (seg_off - lead);
+  uint8_t const* seg_base = a.blocks + size_t(row0) * row_stride + (seg_off - lead);
   auto issue_pair = [&](int pair, uint32_t dst, uint32_t bar) {
     uint8_t const* src = seg_base + size_t(2 * pair) * row_stride;
     bool const two = 2 * pair + 1 < nrows;
@@ -509,15 +500,14 @@ KqPlan const& kq_plan(int n, int bpr, int gy) {
 }
 
 template <int QT>
-bool enqueue_kq1(uint8_t const* blocks, __half const* x, float* out, int const* offsets, int n, int bpr, int experts, int rows,
-                 int max_rows, unsigned int* status, cudaStream_t stream) {
-  int const gy = offsets ? experts * max_rows : rows;
+bool enqueue_kq1(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, unsigned int* status, cudaStream_t stream) {
+  int const gy = rows;
   if (gy <= 0 || gy > 65535) return false;
   KqPlan const& p = kq_plan<QT>(n, bpr, gy);
   if (!p.ok) return false;
   KqArgs a{};
-  a.blocks = blocks; a.x = x; a.out = out; a.offsets = offsets;
-  a.n = n; a.bpr = bpr; a.max_rows = max_rows;
+  a.blocks = blocks; a.x = x; a.out = out;
+  a.n = n; a.bpr = bpr;
   a.S = p.S; a.nbs = p.nbs; a.RS = p.RS; a.seg_stride = p.seg_stride; a.status = status;
   a.rows_q = n / p.gx; a.rows_r = n % p.gx;
   static bool const no_pdl = std::getenv("QUACTLIZE_B200_NO_PDL") != nullptr;
@@ -534,13 +524,13 @@ bool enqueue_kq1(uint8_t const* blocks, __half const* x, float* out, int const* 
 }  // namespace
 
 // Enqueue; false when the format or the shape is outside this kernel's envelope (the caller then uses another kernel).
-bool enqueue_kquant_gemv1(uint8_t const* blocks, __half const* x, float* out, int const* offsets, int n, int bpr, int experts,
-                          int rows, int max_rows, int qtype, unsigned int* status, cudaStream_t stream) {
+bool enqueue_kquant_gemv1(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, int qtype, unsigned int* status,
+                          cudaStream_t stream) {
   switch (qtype) {
-    case 10: return enqueue_kq1<10>(blocks, x, out, offsets, n, bpr, experts, rows, max_rows, status, stream);
-    case 11: return enqueue_kq1<11>(blocks, x, out, offsets, n, bpr, experts, rows, max_rows, status, stream);
-    case 13: return enqueue_kq1<13>(blocks, x, out, offsets, n, bpr, experts, rows, max_rows, status, stream);
-    case 14: return enqueue_kq1<14>(blocks, x, out, offsets, n, bpr, experts, rows, max_rows, status, stream);
+    case 10: return enqueue_kq1<10>(blocks, x, out, n, bpr, rows, status, stream);
+    case 11: return enqueue_kq1<11>(blocks, x, out, n, bpr, rows, status, stream);
+    case 13: return enqueue_kq1<13>(blocks, x, out, n, bpr, rows, status, stream);
+    case 14: return enqueue_kq1<14>(blocks, x, out, n, bpr, rows, status, stream);
     default: return false;
   }
 }

@@ -135,19 +135,19 @@ int enqueue_native_gemv(uint8_t const* blocks, __half const* x, float* out, int 
     //   two rows, few output rows: Q5_K n = 2400 6.6 against 7.3, n = 4800 9.3 against 9.3; a 2048-deep Q6_K 8.0 against 6.5
     //   Q2_K, the fewest bytes: 13.3 against 14.6 for two rows also at n = 14336
     //   three rows: Q5_K n = 1024 5.2 against 5.9, n = 2400 7.9 against 7.3
-    bool one_row = m_rows == 1 || (bpr >= 16 && ((m_rows == 2 && (qtype == 10 || tiles <= sms)) || (m_rows == 3 && 2 * tiles <= sms)));
-    // ragged, at most two rows per expert and many weights: Q4_K 48 against 57, Q2_K 52 against 64 (12 rows, 32 experts,
-    // n = 8192; the formats with more arithmetic per code are faster in one pass); with few weights the empty (expert, row)
-    // CTAs of the one-row launch cost more than they save: 13.6 against 8.9 (one row, 8 experts, n = 4096)
-    if (offsets) one_row = rows_hint <= 2 && (qtype == 10 || qtype == 12) && (long long)m_rows * tiles >= 32ll * sms;
+    // Ragged launches always share: their offsets need not have been checked there, the call then has one kernel whatever the
+    // type of its activations and its offsets, and sums stay fp32.  At most two rows per expert, one row per pass against it:
+    // 2048-deep Q4_K, 12 rows of 32 experts, n = 8192 45.8 against 33.5, 64 rows of 128 experts, n = 1536 66.5 against 34.4; 4096-deep
+    // 46.6 against 46.5, and 6 rows of 8 experts, n = 14336 39 against 45.
+    bool const one_row = !offsets && (m_rows == 1 || (bpr >= 16 && ((m_rows == 2 && (qtype == 10 || tiles <= sms)) || (m_rows == 3 && 2 * tiles <= sms))));
     if (qtype == 12 && !offsets && m_rows >= 2 && m_rows <= 4 && bpr <= 16 && tiles <= 3 * sms) {
       // two to four Q4_K rows, few tiles per SM: no copy and reducing warps to start and drain (5.9 against 6.05 us at
       // n = 2400, 7.4 against 7.6 at 4800, 13.7 against 13.0 at 14336)
       if (enqueue_q4k_rows(blocks, x, out, n, bpr, m_rows, a.status, stream)) return 0;
     }
     if (one_row && aligned) {
-      if (qtype == 12 ? enqueue_q4k_gemv1(blocks, x, out, offsets, n, bpr, a.experts, m_rows, max_rows, a.status, stream)
-                      : enqueue_kquant_gemv1(blocks, x, out, offsets, n, bpr, a.experts, m_rows, max_rows, qtype, a.status, stream)) return 0;
+      if (qtype == 12 ? enqueue_q4k_gemv1(blocks, x, out, n, bpr, m_rows, a.status, stream)
+                      : enqueue_kquant_gemv1(blocks, x, out, n, bpr, m_rows, qtype, a.status, stream)) return 0;
     }
     // Everything else, rows off a 16-byte boundary among it (K % 2048 != 0 for Q3_K and Q6_K, K % 1024 != 0 for Q2_K), which
     // the plain kernel took 67-141 us for at 14336 x 4096.

@@ -34,8 +34,7 @@ struct Q4Args {
   uint8_t const* blocks;
   __half const* x;
   float* out;
-  int const* offsets;        // cumulative [experts+1] (grouped) or nullptr (dense)
-  int n, bpr, max_rows;      // grid.y = activation rows (dense) or experts*max_rows (grouped)
+  int n, bpr;                // grid.y = activation rows
   int S, nbs, RS, iters;     // K segments per row, blocks per segment, row slots per CTA, rows per slot
   int rows_q, rows_r;        // n = gridDim.x*rows_q + rows_r: CTA c owns rows_q (+1 if c < rows_r) consecutive rows
   unsigned int* status;
@@ -151,18 +150,10 @@ __global__ void __launch_bounds__(kQ4Warps * 32, 1) q4k_gemv1_kernel(Q4Args a) {
   // the warp index is broadcast from lane 0 so the compiler keeps everything derived from it in uniform registers
   int const T = blockDim.x, W = T >> 5, warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   int const seg = warp % a.S, rslot = warp / a.S;
-  int e = 0, arow;
-  // Under programmatic dependent launch the offsets and the activation may be the preceding kernel's output: nothing
-  // of them is read before this wait (it also precedes the early return of surplus CTAs).
+  int const arow = blockIdx.y;
+  // Under programmatic dependent launch the activation may be the preceding kernel's output: nothing of it is read before
+  // this wait.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (a.offsets) {
-    e = blockIdx.y / a.max_rows;
-    int const r = blockIdx.y % a.max_rows, r0 = a.offsets[e], r1 = a.offsets[e + 1];
-    if (r >= r1 - r0) return;                                   // uniform for the CTA
-    arow = r0 + r;
-  } else {
-    arow = blockIdx.y;
-  }
 #if defined(QB_ABL_EMPTY)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0 && blockIdx.x == 0) a.out[0] = 1.f;
@@ -208,9 +199,9 @@ __global__ void __launch_bounds__(kQ4Warps * 32, 1) q4k_gemv1_kernel(Q4Args a) {
   // does not change the row's arithmetic, so results do not depend on the claiming order.
   static_assert(STAGES == 2, "the claim bookkeeping below keeps two pairs per warp");
   size_t const seg_off = size_t(seg) * a.nbs * 144;
-  // the row's segment in memory: rows of the first matrix (of expert e), then, for a two-matrix launch, of the second
+  // the row's segment in memory: rows of the first matrix, then, for a two-matrix launch, of the second
   auto row_src = [&](int grow) -> uint8_t const* {
-    return grow < a.n_first ? a.blocks + (size_t(e) * a.n_first + size_t(grow)) * row_stride + seg_off
+    return grow < a.n_first ? a.blocks + size_t(grow) * row_stride + seg_off
                             : a.blocks2 + size_t(grow - a.n_first) * row_stride + seg_off;
   };
   auto issue_pair = [&](int pair, uint32_t dst, uint32_t bar) {
@@ -428,15 +419,15 @@ Q4Plan1 const& q4k_plan1(int n, int bpr, int gy) {
 }  // namespace
 
 // Enqueue; false when the shape is outside this kernel's envelope (the caller then uses another kernel).
-bool enqueue_q4k_gemv1(uint8_t const* blocks, __half const* x, float* out, int const* offsets, int n, int bpr,
-                       int experts, int rows, int max_rows, unsigned int* status, cudaStream_t stream) {
-  int const gy = offsets ? experts * max_rows : rows;
+bool enqueue_q4k_gemv1(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, unsigned int* status,
+                       cudaStream_t stream) {
+  int const gy = rows;
   if (gy <= 0 || gy > 65535) return false;
   Q4Plan1 const& p = q4k_plan1(n, bpr, gy);
   if (!p.ok) return false;
   Q4Args a{};
-  a.blocks = blocks; a.x = x; a.out = out; a.offsets = offsets;
-  a.n = n; a.bpr = bpr; a.max_rows = max_rows;
+  a.blocks = blocks; a.x = x; a.out = out;
+  a.n = n; a.bpr = bpr;
   a.blocks2 = nullptr; a.out2 = nullptr; a.n_first = n;
   a.S = p.S; a.nbs = p.nbs; a.RS = p.RS; a.iters = p.iters; a.status = status;
   a.rows_q = n / p.gx; a.rows_r = n % p.gx;
@@ -460,8 +451,8 @@ bool enqueue_q4k_gemv1_dual(uint8_t const* blocks1, int n1, uint8_t const* block
   Q4Plan1 const& p = q4k_plan1(n1 + n2, bpr, 1);
   if (!p.ok) return false;
   Q4Args a{};
-  a.blocks = blocks1; a.x = x; a.out = out1; a.offsets = nullptr;
-  a.n = n1 + n2; a.bpr = bpr; a.max_rows = 1;
+  a.blocks = blocks1; a.x = x; a.out = out1;
+  a.n = n1 + n2; a.bpr = bpr;
   a.blocks2 = blocks2; a.out2 = out2; a.n_first = n1;
   a.S = p.S; a.nbs = p.nbs; a.RS = p.RS; a.iters = p.iters; a.status = status;
   a.rows_q = a.n / p.gx; a.rows_r = a.n % p.gx;

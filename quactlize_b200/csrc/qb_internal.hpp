@@ -11,14 +11,14 @@ namespace qb {
 int enqueue_native_gemv(uint8_t const* blocks, __half const* x, float* out, int const* offsets,
                         int n, int bpr, int experts, int m_rows, int max_rows, int qtype, bool per_row_x,
                         bool force_generic, cudaStream_t stream);
-bool enqueue_q4k_gemv1(uint8_t const* blocks, __half const* x, float* out, int const* offsets, int n, int bpr,
-                       int experts, int rows, int max_rows, unsigned int* status, cudaStream_t stream);
+bool enqueue_q4k_gemv1(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, unsigned int* status,
+                       cudaStream_t stream);                // dense, one activation row per pass over the weights
 bool enqueue_q4k_gemv1_dual(uint8_t const* blocks1, int n1, uint8_t const* blocks2, int n2, __half const* x, float* out1, float* out2,
                             int bpr, unsigned int* status, cudaStream_t stream);   // two matrices, one activation row, one launch
 bool enqueue_q4k_rows(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, unsigned int* status,
                       cudaStream_t stream);                 // dense, 1..8 rows, tensor cores on the single-row kernel's copy structure
-bool enqueue_kquant_gemv1(uint8_t const* blocks, __half const* x, float* out, int const* offsets, int n, int bpr, int experts,
-                          int rows, int max_rows, int qtype, unsigned int* status, cudaStream_t stream);   // Q2_K/Q3_K/Q5_K/Q6_K, one row per pass
+bool enqueue_kquant_gemv1(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, int qtype, unsigned int* status,
+                          cudaStream_t stream);             // Q2_K/Q3_K/Q5_K/Q6_K, dense, one row per pass
 bool enqueue_kq_rows(uint8_t const* blocks, __half const* x, float* out, int const* offsets, int n, int bpr, int experts, int rows,
                      int qtype, unsigned int* status, cudaStream_t stream);   // every k-quant, up to eight rows per weight pass, dense and ragged
 bool enqueue_dequantize(uint8_t const* blocks, __half* out, int count, int qtype, cudaStream_t s);

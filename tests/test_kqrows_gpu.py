@@ -62,6 +62,24 @@ def test_blocks_off_a_16_byte_boundary(qt):
         assert kq.max_rel(out, want) < 2e-5, shift
 
 
+@pytest.mark.parametrize("e,n,k,rows", [(64, 1184, 256, 64), (1500, 33, 512, 40)])
+@pytest.mark.parametrize("qt", [10, 12])
+def test_moe_takes_one_kernel_whoever_asks(qt, e, n, k, rows):
+    """At most two rows per expert and many tiles, or many experts: the native call, the converting one and the C ABI agree to the
+    last bit, and sums are fp32."""
+    blocks = synth.kquant_blocks(qt, e * n * k // 256, seed=qt).reshape(e, n * k // 256, -1)
+    x = synth.activations(rows, k, seed=3)
+    off = np.concatenate([[0], np.cumsum(np.random.default_rng(e).permutation([1] * rows + [0] * (e - rows)))]).astype(np.int32)
+    b, xx, o = _cuda(blocks), _cuda(x), _cuda(off)
+    native = qb.gguf_vecdot_moe(b, xx, o, qt)
+    assert torch.equal(native, qb.gguf_vecdot_moe(b, xx.float(), o, qt))
+    out = torch.empty((rows, n), device=DEV)
+    rc = _lib.lib().quactlize_b200_vecdot_moe_dev_v1(b.data_ptr(), b.shape[2], xx.data_ptr(), o.data_ptr(), out.data_ptr(), n, k // 256, e, rows, 1, qt,
+                                                     torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and torch.equal(native, out)
+    assert kq.max_rel(native.cpu().numpy(), kq.vecdot_moe(blocks, x, off, n, k, qt)) < 2e-5
+
+
 def test_moe_refuses_bad_offsets():
     """Offsets that do not describe the rows raise, whatever was enqueued meanwhile, and the next call is right."""
     e, n, k = 3, 64, 1024
