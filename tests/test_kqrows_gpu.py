@@ -35,6 +35,14 @@ def test_rows(qt, m, n, k):
     assert kq.max_rel(out, ref) < (4e-3 if fp16_sums else 2e-5)
 
 
+@pytest.mark.parametrize("m,n,k", [(2, 500, 8192), (3, 200, 14336), (2, 100, 4352)])
+def test_q4k_sums_stay_fp32_on_deep_rows(m, n, k):
+    blocks = synth.kquant_blocks(12, n * k // 256, seed=m)
+    x = synth.activations(m, k, seed=n)
+    out = qb.gguf_vecdot_rows(_cuda(blocks), _cuda(x), n, k, 12).cpu().numpy()
+    assert kq.max_rel(out, np.concatenate([kq.vecdot_dense(blocks, x[i:i + 1], n, k, 12).reshape(1, n) for i in range(m)])) < 2e-5
+
+
 @pytest.mark.parametrize("counts", [[0, 0, 1, 0], [3, 0, 17, 8, 1], [1] * 16, [0, 9, 0, 0, 0, 0, 2]])
 @pytest.mark.parametrize("n,k", [(70, 768), (300, 2304), (40, 8448)])
 @pytest.mark.parametrize("qt", QTYPES)
