@@ -421,6 +421,29 @@ __device__ __forceinline__ void kr_compute(KrArgs const& a, KrWalk wk, int const
   }
 }
 
+// A ring stage of a tile at an end of the tensor [lo, hi) that is off a 16-byte boundary (rare, and kept out of the copy warp's loop).
+__device__ __noinline__ void kr_copy_ends(uint8_t* stage, int pitch, uintptr_t b0, size_t step, int rows, unsigned len, uintptr_t lo, uintptr_t hi,
+                                          uint64_t* full, int lane) {
+  unsigned total = 0;
+  for (int r = lane; r < rows; r += 32) {
+    uintptr_t const b = b0 + size_t(r) * step;
+    KrSpan const s = kr_span(b, len, lo, hi);
+    uint8_t* const dst = stage + size_t(r) * pitch;
+    total += unsigned(s.to - s.from);
+    for (uintptr_t p = b; p < s.from; ++p) dst[p - s.first] = __ldg(reinterpret_cast<uint8_t const*>(p));
+    for (uintptr_t p = s.to; p < b + len; ++p) dst[p - s.first] = __ldg(reinterpret_cast<uint8_t const*>(p));
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  total = __reduce_add_sync(0xffffffffu, total);                    // and the bytes are written before lane 0 arrives
+  __syncwarp();
+  if (lane == 0) mbar_expect_tx(full, total);
+  __syncwarp();
+  for (int r = lane; r < rows; r += 32) {
+    KrSpan const s = kr_span(b0 + size_t(r) * step, len, lo, hi);
+    bulk_g2s(stage + size_t(r) * pitch + (s.from - s.first), reinterpret_cast<void const*>(s.from), unsigned(s.to - s.from), full);
+  }
+}
+
 template <int QT>
 __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
   constexpr int kBytes = kq::Fmt<QT>::kBytes;
@@ -503,6 +526,7 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
     // ---- copies ---------------------------------------------------------------------------------------------------------
     KrRing ws{}, xr{};
     uintptr_t const lo = reinterpret_cast<uintptr_t>(a.blocks), hi = lo + size_t(a.offsets ? a.experts : 1) * a.n * a.bpr * kBytes;
+    bool const odd_ends = ((lo | hi) & 15u) != 0;
     bool first = a.xrows <= kKrDirectRows;                          // the computing warps load these activations themselves
     while (!dead && wk.next(a, offp, cum)) {
       for (int p = 0; p < a.passes && !dead; ++p) {
@@ -523,28 +547,25 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
           if (ws.lap && !mbar_wait_bounded(&bar->empty[ws.i], ws.phase ^ 1u, a.status, kWaitStageTimeout)) { dead = true; break; }
           int const rows = nb ? min(min(a.RS, wk.t1 - tb) * kKrTile, a.n - tb * kKrTile) : 0;
           uint8_t* const stage = ring + ws.i * stage_bytes;
-          auto span = [&](int r) { return kr_span(reinterpret_cast<uintptr_t>(src0 + size_t(r) * step), len, lo, hi); };
-          unsigned total = 0;
-          for (int r = lane; r < rows; r += 32) {
-            KrSpan const s = span(r);
-            total += unsigned(s.to - s.from);
-            if constexpr (QT != 12 && QT != 13) {                   // the ends of the tensor, off a 16-byte boundary
-              uintptr_t const b = reinterpret_cast<uintptr_t>(src0 + size_t(r) * step);
-              if (s.from > b || s.to < b + len) {
-                uint8_t* const dst = stage + size_t(r) * a.pitch;
-                for (uintptr_t p = b; p < s.from; ++p) dst[p - s.first] = __ldg(reinterpret_cast<uint8_t const*>(p));
-                for (uintptr_t p = s.to; p < b + len; ++p) dst[p - s.first] = __ldg(reinterpret_cast<uint8_t const*>(p));
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-              }
-            }
+          // a tensor that begins or ends inside a 16-byte unit: its first and last tiles are copied with that in mind
+          if (QT != 12 && QT != 13 && odd_ends && (tb == 0 || tb + a.RS >= a.tiles)) {
+            kr_copy_ends(stage, a.pitch, reinterpret_cast<uintptr_t>(src0), step, rows, len, lo, hi, &bar->full[ws.i], lane);
+            continue;
           }
+          auto span = [&](int r, uint8_t const*& from) -> unsigned {    // the 16-byte units that hold row r's segment
+            uintptr_t const b = reinterpret_cast<uintptr_t>(src0 + size_t(r) * step);
+            from = reinterpret_cast<uint8_t const*>(b & ~uintptr_t(15));
+            return unsigned(((b + len + 15) & ~uintptr_t(15)) - (b & ~uintptr_t(15)));
+          };
+          unsigned total = 0;
+          uint8_t const* from;
+          for (int r = lane; r < rows; r += 32) total += span(r, from);
           total = __reduce_add_sync(0xffffffffu, total);
-          __syncwarp();                                             // the bytes are written before lane 0 arrives
           if (lane == 0) mbar_expect_tx(&bar->full[ws.i], total);
           __syncwarp();
           for (int r = lane; r < rows; r += 32) {
-            KrSpan const s = span(r);
-            bulk_g2s(stage + size_t(r) * a.pitch + (s.from - s.first), reinterpret_cast<void const*>(s.from), unsigned(s.to - s.from), &bar->full[ws.i]);
+            unsigned const bytes = span(r, from);
+            bulk_g2s(stage + size_t(r) * a.pitch, from, bytes, &bar->full[ws.i]);
           }
         }
       }
