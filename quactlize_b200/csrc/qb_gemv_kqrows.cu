@@ -11,8 +11,17 @@
 // subnormals q * 2^-24) times the sub-scale is an A fragment of mma.sync.m16n8k16 and all 256 codes of a superblock go
 // into one fp32 accumulator tile, scaled by d once.  The B fragments are the fp16 activations as they are.  Which code
 // feeds which k index is free as long as A and B agree, so a lane reads its own 16-byte chunk of a weight row and needs
-// the sub-scales of four groups only, with no exchange between lanes.  Sub-mins: one (Q2_K: two) tf32 MMA against the
-// per-group sums of x, the sums split in two tf32 halves (22 bits); the sums come from 16 MMAs with an indicator matrix.
+// the sub-scales of four groups only, with no exchange between lanes.  Sub-mins: two (Q2_K: three) bf16 MMAs against the
+// per-group sums of x, the fp32 sums whole as three bf16 parts of 8 bits; the sums come from 16 MMAs with an indicator matrix.
+//
+// Rounding.  An MMA cuts its fp32 sum off where a fused multiply-add rounds, and it lines its products up by their exponent
+// fields, so an fp16 subnormal costs the sum as many bits as it has leading zeros.  The sub-scales therefore carry a power of two
+// (kr_up) that lifts the products out of the subnormals, a chain of MMAs is at most four long before its sum goes to a rounded
+// add, and a tile's K slices are added even and odd apart.  Relative error against 64 bits, N(0,1) activations, K 1280 to
+// 14336, against 22-bit group sums, chains of eight (Q6_K sixteen) and no lift: Q2_K 2.2e-7 -> 0.8e-7, Q3_K 1.2e-7 -> 0.8e-7, Q4_K 1.8e-7 ->
+// 1.2e-7, Q5_K 2.0e-7 -> 1.3e-7; 4096 -> 14336, us: Q2_K 8 rows 14.9 -> 13.1, Q3_K 4 rows 15.9 -> 16.2, Q4_K 8 rows 13.2 -> 13.0, Q5_K 4 rows 16.3 -> 16.2.  Q6_K, two products a code, has its chains cut only where a rounded kernel
+// was before it: rows off a 16-byte boundary 2.3e-7 -> 1.0e-7 (4096 x 2304, three rows 8.0 -> 9.0 us; the plain kernel 0.8e-7 and 38 us);
+// its other rows took the one-row kernel's 8e-4 before and keep 2.3e-7.
 //
 // Structure.  One CTA per SM: 16 computing warps, a copy warp, a reducing warp.  K is covered in passes of P superblocks,
 // and for deep rows cut over the CTAs of a cluster; warp (slot, b) owns superblock b of the pass and keeps its B fragments
@@ -28,6 +37,7 @@
 // Measured, 4096 -> 14336, eight rows, us: Q4_K 15.5 -> 13.4 (33 MB, 2.5 TB/s), Q2_K 41 -> 14.8, Q3_K 64 -> 16.6, Q5_K 58 -> 15.9,
 // Q6_K 66 -> 19.6.  What bounds it is the latency of a tile round, 1.13 us for Q4_K against 0.83 us of stream: about 260
 // instructions a warp, half of them on the half-rate integer pipe, with four to five warps per scheduler.
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -80,20 +90,31 @@ __device__ __forceinline__ void kr_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void kr_mma_tf32(float (&c)[4], float const (&a)[4], float b0, float b1) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
-                 "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+// D = A * B: the first of a chain
+__device__ __forceinline__ void kr_mma0(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
+__device__ __forceinline__ void kr_mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void kr_mma_bf16_k8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
+}
+// power of two on the scaled codes: the largest whose constant in kr_scale is an fp16 number, with 16 * sc in Q6_K's range
+template <int QT> constexpr float kr_up() { return QT == 14 ? 16.f : 32.f; }
 __device__ __forceinline__ __half2 kr_mask(uint32_t w, uint32_t m) { return u32_as_h2(w & m); }
 // byte `idx` of w, as half2 (b + add) * mul in both lanes; exact for the values used here
 __device__ __forceinline__ __half2 kr_scale(uint32_t w, uint32_t idx, float mul, float add) {
   return __hfma2(u32_as_h2(__byte_perm(w, 0x64646464u, 0x4040u + 0x0101u * idx)), __float2half2_rn(mul), __float2half2_rn((add - 1024.f) * mul));
 }
-// byte `idx` of w as a float
-__device__ __forceinline__ float kr_byte_f(uint32_t w, uint32_t idx) {
-  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + idx)) - 8388608.f;
+// bytes 2p, 2p+1 of w, below 128, as a bf16 pair: 128 + b has b in its mantissa
+__device__ __forceinline__ uint32_t kr_min_pair(uint32_t w, uint32_t p) {
+  uint32_t v = __byte_perm(w, 0x43434343u, 0x4140u + 0x0202u * p);
+  __nv_bfloat162 const m = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&v), __float2bfloat162_rn(128.f));
+  return *reinterpret_cast<uint32_t const*>(&m);
 }
 
 // One weight row's share of a lane: the words, one sub-scale multiplier per field, the header.  load() reads it; frag(j, wi)
@@ -103,7 +124,8 @@ template <int QT> struct KrRow;
 template <> struct KrRow<12> {                                      // Q4_K
   uint32_t q[2][4];
   __half2 s[4];
-  float d, dmin, mn[2];
+  float d, dmin;
+  uint32_t mn[1];                                                   // sub-mins of groups 2t, 2t+1
   __device__ __forceinline__ void load(uint32_t sb, int t) {
     uint4 const h = kr_lds128(sb);
     codes(sb + 16 + 16 * t);
@@ -120,9 +142,10 @@ template <> struct KrRow<12> {                                      // Q4_K
     uint32_t const sc_lo = h.y & 0x3F3F3F3Fu, sc_hi = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
     uint32_t const mn_lo = h.z & 0x3F3F3F3Fu, mn_hi = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
     uint32_t const i0 = uint32_t(t & 2);                            // the chunk's even group within its word
-    s[0] = kr_scale(sc_lo, i0, 1.f, 0.f); s[1] = kr_scale(sc_lo, i0 + 1, 0.0625f, 0.f);
-    s[2] = kr_scale(sc_hi, i0, 1.f, 0.f); s[3] = kr_scale(sc_hi, i0 + 1, 0.0625f, 0.f);
-    mn[0] = kr_byte_f(mn_lo, t); mn[1] = kr_byte_f(mn_hi, t);
+    constexpr float up = kr_up<12>();
+    s[0] = kr_scale(sc_lo, i0, up, 0.f); s[1] = kr_scale(sc_lo, i0 + 1, up * 0.0625f, 0.f);
+    s[2] = kr_scale(sc_hi, i0, up, 0.f); s[3] = kr_scale(sc_hi, i0 + 1, up * 0.0625f, 0.f);
+    mn[0] = kr_min_pair((t & 2) ? mn_hi : mn_lo, uint32_t(t & 1));
   }
   __device__ __forceinline__ void frag(int j, int wi, uint32_t (&a)[2]) const {
     uint32_t const w = q[j >> 1][wi], m = (j & 1) ? 0x00F000F0u : 0x000F000Fu;
@@ -154,7 +177,8 @@ template <> struct KrRow<13> : KrRow<12> {                          // Q5_K: the
 template <> struct KrRow<10> {                                      // Q2_K (4-byte aligned blocks)
   uint32_t q[4];
   __half2 s[4];
-  float d, dmin, mn[4];
+  float d, dmin;
+  uint32_t mn[2];                                                   // sub-mins of groups 2t, 2t+1 and 2t+8, 2t+9
   __device__ __forceinline__ void load(uint32_t sb, int t) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) q[i] = kr_lds32(sb + 16 + 16 * t + 4 * ((i + t) & 3));
@@ -162,10 +186,11 @@ template <> struct KrRow<10> {                                      // Q2_K (4-b
     float2 const dd = __half22float2(u32_as_h2(kr_lds32(sb + 80)));
     d = dd.x; dmin = dd.y;
     uint32_t const sa = ((t & 2) ? w2 : w0) & 0x0F0F0F0Fu, sc = ((t & 2) ? w3 : w1) & 0x0F0F0F0Fu, p = uint32_t(t & 1);
-    s[0] = kr_scale(sa, p, 1.f, 0.f);        s[1] = kr_scale(sa, p + 2, 0.25f, 0.f);
-    s[2] = kr_scale(sc, p, 0.0625f, 0.f);    s[3] = kr_scale(sc, p + 2, 0.015625f, 0.f);
-    mn[0] = kr_byte_f((w0 >> 4) & 0x0F0F0F0Fu, t); mn[1] = kr_byte_f((w1 >> 4) & 0x0F0F0F0Fu, t);
-    mn[2] = kr_byte_f((w2 >> 4) & 0x0F0F0F0Fu, t); mn[3] = kr_byte_f((w3 >> 4) & 0x0F0F0F0Fu, t);
+    constexpr float up = kr_up<10>();
+    s[0] = kr_scale(sa, p, up, 0.f);              s[1] = kr_scale(sa, p + 2, up * 0.25f, 0.f);
+    s[2] = kr_scale(sc, p, up * 0.0625f, 0.f);    s[3] = kr_scale(sc, p + 2, up * 0.015625f, 0.f);
+    mn[0] = kr_min_pair((((t & 2) ? w1 : w0) >> 4) & 0x0F0F0F0Fu, p);
+    mn[1] = kr_min_pair((((t & 2) ? w3 : w2) >> 4) & 0x0F0F0F0Fu, p);
   }
   __device__ __forceinline__ void frag(int j, int wi, uint32_t (&a)[2]) const {
     uint32_t const m = 0x00030003u << (2 * j);
@@ -200,8 +225,9 @@ template <> struct KrRow<11> {                                      // Q3_K (2-b
     d = __half2float(__ushort_as_half(uint16_t(kr_lds16(sb + 108))));
     uint32_t const lo = (a0 & 0x0F0F0F0Fu) | ((a2 & 0x03030303u) << 4), hi = (a1 & 0x0F0F0F0Fu) | (((a2 >> 2) & 0x03030303u) << 4);
     uint32_t const p = uint32_t(t & 1);
-    s[0] = kr_scale(lo, p, 1.f, -32.f);      s[1] = kr_scale(lo, p + 2, 0.25f, -32.f);
-    s[2] = kr_scale(hi, p, 0.0625f, -32.f);  s[3] = kr_scale(hi, p + 2, 0.015625f, -32.f);
+    constexpr float up = kr_up<11>();
+    s[0] = kr_scale(lo, p, up, -32.f);            s[1] = kr_scale(lo, p + 2, up * 0.25f, -32.f);
+    s[2] = kr_scale(hi, p, up * 0.0625f, -32.f);  s[3] = kr_scale(hi, p + 2, up * 0.015625f, -32.f);
     sn[0] = __hmul2(s[0], __float2half2_rn(-4.f)); sn[1] = __hmul2(s[1], __float2half2_rn(-8.f));       // -4*sc / 2^j
     sn[2] = __hmul2(s[2], __float2half2_rn(-16.f)); sn[3] = __hmul2(s[3], __float2half2_rn(-32.f));
   }
@@ -226,8 +252,9 @@ template <> struct KrRow<14> {                                      // Q6_K (2-b
     uint32_t const lo = __funnelshift_r(v0, v1, shf) ^ 0x80808080u, hi = __funnelshift_r(v1, v2, shf) ^ 0x80808080u;
     d = __half2float(__ushort_as_half(uint16_t(kr_lds16(sb + 208))));
     uint32_t const p = uint32_t(t & 1);
-    __half2 const c0 = kr_scale(lo, p, 1.f, -128.f), c1 = kr_scale(lo, p + 2, 1.f, -128.f);
-    __half2 const c2 = kr_scale(hi, p, 1.f, -128.f), c3 = kr_scale(hi, p + 2, 1.f, -128.f);
+    constexpr float up = kr_up<14>();
+    __half2 const c0 = kr_scale(lo, p, up, -128.f), c1 = kr_scale(lo, p + 2, up, -128.f);
+    __half2 const c2 = kr_scale(hi, p, up, -128.f), c3 = kr_scale(hi, p + 2, up, -128.f);
     __half2 const sixteenth = __float2half2_rn(0.0625f), off = __float2half2_rn(-0x1p-19f);             // -32 * 2^-24
     s[0] = c0; s[1] = c1; s[2] = __hmul2(c2, sixteenth); s[3] = __hmul2(c3, sixteenth);
     sh[0] = __hmul2(c0, __float2half2_rn(16.f)); sh[1] = __hmul2(c1, __float2half2_rn(4.f));            // 16*sc / 4^j
@@ -289,12 +316,13 @@ struct KrRing {
 struct KrBars { uint64_t full[kKrMaxStages], empty[kKrMaxStages], xfull[2], xempty[2], pfull[2], pempty[2], cfull; };
 
 // One computing warp: its superblock of every tile of the CTA.
-template <int QT>
+template <int QT, bool FINE>
 __device__ __forceinline__ void kr_compute(KrArgs const& a, KrWalk wk, int const* offp, int const* cum, uint8_t* ring, uint8_t* xs, float* part,
                                            KrBars* bar, uint32_t stage_bytes, int warp, int lane, int k0) {
   constexpr int kBytes = kq::Fmt<QT>::kBytes;
   constexpr bool kHasMin = kq::Fmt<QT>::kHasMin;
-  constexpr int kMin = QT == 10 ? 4 : 2;                            // sub-mins per lane and row
+  constexpr int kMin = QT == 10 ? 2 : 1;                            // pairs of sub-mins per lane and row
+  constexpr int kChain = QT == 14 ? (FINE ? 2 : 8) : 4;             // fragments of a chain
   bool dead = false;
   int const g = lane >> 2, t = lane & 3;
   int const slot = warp / a.P, b = warp - slot * a.P;
@@ -335,7 +363,7 @@ __device__ __forceinline__ void kr_compute(KrArgs const& a, KrWalk wk, int const
         uint32_t const lo = bf[i][0], hi = bf[i][1];
         bf[i][0] = __byte_perm(lo, hi, 0x5410); bf[i][1] = __byte_perm(lo, hi, 0x7632);
       }
-      float bs[kHasMin ? kMin : 1][2];                              // group sums: B registers of the sub-min MMAs, two tf32 halves
+      uint32_t bs[3][kMin];                                         // group sums: B registers of the sub-min MMAs, three bf16 parts
       if constexpr (kHasMin) {
         float c4[4][4] = {};                                        // four chains: an MMA waits for the one before it
 #pragma unroll
@@ -347,15 +375,22 @@ __device__ __forceinline__ void kr_compute(KrArgs const& a, KrWalk wk, int const
         float c[4];                                                 // the chains are different groups: all but one are zero
 #pragma unroll
         for (int i = 0; i < 4; ++i) c[i] = (c4[0][i] + c4[1][i]) + (c4[2][i] + c4[3][i]);
-        // row = group, column = activation row -> k index = group (t, t+4 and, with 16 groups, t+8, t+12), column g
-        int const src = t * 4 + (g >> 1);
+        // row = group, column = activation row -> k index = group (2t, 2t+1 and, with 16 groups, 2t+8, 2t+9), column g
 #pragma unroll
-        for (int i = 0; i < kMin; ++i) {
-          float const e0 = __shfl_sync(0xffffffffu, c[2 * (i >> 1)], src + 16 * (i & 1));
-          float const e1 = __shfl_sync(0xffffffffu, c[2 * (i >> 1) + 1], src + 16 * (i & 1));
-          float const v = (g & 1) ? e1 : e0;
-          bs[i][0] = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
-          bs[i][1] = v - bs[i][0];
+        for (int h = 0; h < kMin; ++h) {
+          float v[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            int const src = 4 * (2 * t + i) + (g >> 1);
+            float const e0 = __shfl_sync(0xffffffffu, c[2 * h], src), e1 = __shfl_sync(0xffffffffu, c[2 * h + 1], src);
+            v[i] = (g & 1) ? e1 : e0;
+          }
+#pragma unroll
+          for (int part = 0; part < 3; ++part) {
+            bs[part][h] = __byte_perm(__float_as_uint(v[0]), __float_as_uint(v[1]), 0x7632);
+            v[0] -= __uint_as_float(__float_as_uint(v[0]) & 0xFFFF0000u);
+            v[1] -= __uint_as_float(__float_as_uint(v[1]) & 0xFFFF0000u);
+          }
         }
       }
       uint32_t mis = 0, mis_step = 0;                               // rows of Q4_K and Q5_K are 16-byte aligned
@@ -373,33 +408,45 @@ __device__ __forceinline__ void kr_compute(KrArgs const& a, KrWalk wk, int const
           KrRow<QT> r0, r1;
           r0.load(base + (mis & 15u), t);
           r1.load(base + 8u * a.pitch + ((mis + 8u * row_step) & 15u), t);
-          float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f}, cm[4] = {0.f, 0.f, 0.f, 0.f};
-          if constexpr (kHasMin) {
+          float cm[4] = {0.f, 0.f, 0.f, 0.f};                       // smallest part first
+          if constexpr (QT == 10) {
 #pragma unroll
-            for (int i = 0; i < kMin; i += 2) {
-              float const am[4] = {r0.mn[i], r1.mn[i], r0.mn[i + 1], r1.mn[i + 1]};
-              kr_mma_tf32(cm, am, bs[i][0], bs[i + 1][0]);
-              kr_mma_tf32(cm, am, bs[i][1], bs[i + 1][1]);
-            }
+            for (int part = 2; part >= 0; --part) kr_mma_bf16(cm, r0.mn[0], r1.mn[0], r0.mn[kMin - 1], r1.mn[kMin - 1], bs[part][0], bs[part][kMin - 1]);
+          } else if constexpr (kHasMin) {
+            kr_mma_bf16(cm, r0.mn[0], r1.mn[0], r0.mn[0], r1.mn[0], bs[2][0], bs[1][0]);
+            kr_mma_bf16_k8(cm, r0.mn[0], r1.mn[0], bs[0][0]);
           }
+          float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, p0[4], p1[4];   // even and odd fragments
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             uint32_t f0[2], f1[2];
             r0.frag(i >> 2, i & 3, f0);
             r1.frag(i >> 2, i & 3, f1);
-            if constexpr (QT == 14) {
-              kr_mma(c0, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
+            if constexpr (QT == 14 && !FINE) {                      // low nibbles and high bits apart
+              kr_mma(s0, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
               r0.frag_high(i >> 2, i & 3, f0);
               r1.frag_high(i >> 2, i & 3, f1);
-              kr_mma(c1, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
+              kr_mma(s1, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
             } else {
-              if (i & 1) kr_mma(c1, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
-              else kr_mma(c0, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
+              float (&p)[4] = (i & 1) ? p1 : p0;
+              if ((i >> 1) % kChain == 0) kr_mma0(p, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
+              else kr_mma(p, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
+              if constexpr (QT == 14) {
+                r0.frag_high(i >> 2, i & 3, f0);
+                r1.frag_high(i >> 2, i & 3, f1);
+                kr_mma(p, f0[0], f1[0], f0[1], f1[1], bf[i][0], bf[i][1]);
+              }
+              if ((i >> 1) % kChain == kChain - 1) {
+                float (&s)[4] = (i & 1) ? s1 : s0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[j] = (i >> 1) < kChain ? p[j] : s[j] + p[j];
+              }
             }
           }
-          float const d0 = r0.d * 16777216.f, d1 = r1.d * 16777216.f;
-          o0.x = d0 * (c0[0] + c1[0]); o0.y = d0 * (c0[1] + c1[1]);
-          o1.x = d1 * (c0[2] + c1[2]); o1.y = d1 * (c0[3] + c1[3]);
+          constexpr float down = 16777216.f / kr_up<QT>();
+          float const d0 = r0.d * down, d1 = r1.d * down;
+          o0.x = d0 * (s0[0] + s1[0]); o0.y = d0 * (s0[1] + s1[1]);
+          o1.x = d1 * (s0[2] + s1[2]); o1.y = d1 * (s0[3] + s1[3]);
           if constexpr (kHasMin) {
             o0.x = fmaf(-r0.dmin, cm[0], o0.x); o0.y = fmaf(-r0.dmin, cm[1], o0.y);
             o1.x = fmaf(-r1.dmin, cm[2], o1.x); o1.y = fmaf(-r1.dmin, cm[3], o1.y);
@@ -444,7 +491,8 @@ __device__ __noinline__ void kr_copy_ends(uint8_t* stage, int pitch, uintptr_t b
   }
 }
 
-template <int QT>
+// FINE: short chains for Q6_K (see "Rounding")
+template <int QT, bool FINE>
 __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
   constexpr int kBytes = kq::Fmt<QT>::kBytes;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -600,12 +648,15 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
           int const nt = min(a.RS, wk.t1 - tb);
           for (int sl = 0; sl < nt; ++sl) {
             float4 const* src = reinterpret_cast<float4 const*>(part + (pr.i * kKrWarps + sl * a.P) * kKrTile * kKrCols) + lane;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f), u = v;      // even and odd superblocks
+            auto add = [](float4& to, float4 o) { to.x += o.x; to.y += o.y; to.z += o.z; to.w += o.w; };
 #pragma unroll 8
-            for (int b = 0; b < nb; ++b) {
-              float4 const o = src[b * (kKrTile * kKrCols / 4)];
-              v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+            for (int b = 0; b + 1 < nb; b += 2) {
+              add(v, src[b * (kKrTile * kKrCols / 4)]);
+              add(u, src[(b + 1) * (kKrTile * kKrCols / 4)]);
             }
+            if (nb & 1) add(v, src[(nb - 1) * (kKrTile * kKrCols / 4)]);
+            add(v, u);
             if (keep_sums) {
               float4* keep = reinterpret_cast<float4*>(seg_acc + (tb + sl - wk.t0) * kKrTile * kKrCols) + lane;
               if (p > 0) { float4 const o = *keep; v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
@@ -642,7 +693,7 @@ __global__ void __launch_bounds__(kKrThreads, 1) kq_rows_kernel(KrArgs a) {
       ++seg;
     }
   } else if (warp < active_warps) {
-    kr_compute<QT>(a, wk, offp, cum, ring, xs, part, bar, stage_bytes, warp, lane, k0);
+    kr_compute<QT, FINE>(a, wk, offp, cum, ring, xs, part, bar, stage_bytes, warp, lane, k0);
   }
   if (a.C > 1) {                                                    // a CTA's sums are read by the others until here
     __syncwarp();
@@ -684,7 +735,7 @@ bool kr_layout(KrPlan& p, int xrows, int experts) {
 }
 
 // `units`: tiles of the launch (ragged: those of a router that spreads its rows).  Plans are kept per shape.
-template <int QT>
+template <int QT, bool FINE>
 KrPlan kr_plan(int bpr, int units, int xrows, int experts) {
   int const sms = rt_sm_count();
   int const per_sm = std::min(64, (units + sms - 1) / sms);         // beyond that the split no longer depends on it
@@ -717,13 +768,13 @@ KrPlan kr_plan(int bpr, int units, int xrows, int experts) {
   }
   if (bestp.ok) {
     bestp.slots = sms / bestp.C;
-    bool fine = cudaFuncSetAttribute(kq_rows_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKrSmem)) == cudaSuccess;
+    bool fine = cudaFuncSetAttribute(kq_rows_kernel<QT, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKrSmem)) == cudaSuccess;
     if (fine && bestp.C > 1) {                                      // clusters that the GPCs hold at the same time
       cudaLaunchConfig_t cfg;
       cudaLaunchAttribute at[2];
       kr_launch_config(cfg, at, bestp, unsigned(bestp.slots * bestp.C), nullptr);
       int resident = 0;
-      fine = cudaOccupancyMaxActiveClusters(&resident, kq_rows_kernel<QT>, &cfg) == cudaSuccess && resident > 0;
+      fine = cudaOccupancyMaxActiveClusters(&resident, kq_rows_kernel<QT, FINE>, &cfg) == cudaSuccess && resident > 0;
       bestp.slots = std::min(bestp.slots, resident);
     }
     if (!fine) { (void)cudaGetLastError(); bestp.ok = 0; }
@@ -731,7 +782,7 @@ KrPlan kr_plan(int bpr, int units, int xrows, int experts) {
   return plans.emplace(key, bestp).first->second;
 }
 
-template <int QT>
+template <int QT, bool FINE = false>
 bool launch(KrArgs a, cudaStream_t stream) {
   a.tiles = (a.n + kKrTile - 1) / kKrTile;
   a.xrows = std::min(kKrCols, a.m_rows);
@@ -739,13 +790,13 @@ bool launch(KrArgs a, cudaStream_t stream) {
   if ((long long)most * a.tiles > kKrMaxUnits) return false;
   // a router that spreads r rows over E experts touches about r of them while r is small against E
   int const likely = a.offsets ? std::max(1, std::min(most, int((long long)a.m_rows * a.experts / (a.m_rows + a.experts)))) : most;
-  KrPlan const p = kr_plan<QT>(a.bpr, likely * a.tiles, a.xrows, a.experts);
+  KrPlan const p = kr_plan<QT, FINE>(a.bpr, likely * a.tiles, a.xrows, a.experts);
   if (!p.ok) return false;
   a.passes = p.passes; a.P = p.P; a.RS = p.RS; a.C = p.C; a.pitch = p.pitch; a.xpitch = p.xpitch; a.stages = p.stages; a.xbufs = p.xbufs; a.round = p.round;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
   kr_launch_config(cfg, at, p, unsigned(std::min(p.slots, most * a.tiles) * p.C), stream);
-  if (cudaLaunchKernelEx(&cfg, kq_rows_kernel<QT>, a) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+  if (cudaLaunchKernelEx(&cfg, kq_rows_kernel<QT, FINE>, a) != cudaSuccess) { (void)cudaGetLastError(); return false; }
   return true;
 }
 
@@ -764,7 +815,7 @@ bool enqueue_kq_rows(uint8_t const* blocks, __half const* x, float* out, int con
     case 11: return launch<11>(a, stream);
     case 12: return launch<12>(a, stream);
     case 13: return launch<13>(a, stream);
-    case 14: return launch<14>(a, stream);
+    case 14: return (reinterpret_cast<uintptr_t>(blocks) | size_t(bpr) * 210) % 16 ? launch<14, true>(a, stream) : launch<14>(a, stream);
     default: return false;
   }
 }

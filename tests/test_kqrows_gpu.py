@@ -43,6 +43,19 @@ def test_q4k_sums_stay_fp32_on_deep_rows(m, n, k):
     assert kq.max_rel(out, np.concatenate([kq.vecdot_dense(blocks, x[i:i + 1], n, k, 12).reshape(1, n) for i in range(m)])) < 2e-5
 
 
+@pytest.mark.parametrize("k", [2304, 4352, 13568])
+@pytest.mark.parametrize("qt", QTYPES)
+def test_error_against_64_bits(qt, k):
+    """Eight rows whose blocks start off a 16-byte boundary where the format allows it.  A sum of thousands of fp32 terms in chains of
+    at most eight tensor-core steps and a pairwise tail: two and a half units of 2^-24 of the result's 2-norm."""
+    m, n = 8, 256
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=qt + k)
+    x = np.random.default_rng(k).standard_normal((m, k)).astype(np.float16)
+    want = x.astype(np.float64) @ kq.dequantize_f32(blocks, qt).reshape(n, k).T
+    got = qb.gguf_vecdot_rows(_cuda(blocks), _cuda(x), n, k, qt).cpu().numpy()
+    assert np.linalg.norm(got - want) < 2.5 * 2.0**-24 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("counts", [[0, 0, 1, 0], [3, 0, 17, 8, 1], [1] * 16, [0, 9, 0, 0, 0, 0, 2]])
 @pytest.mark.parametrize("n,k", [(70, 768), (300, 2304), (40, 8448)])
 @pytest.mark.parametrize("qt", QTYPES)
