@@ -734,50 +734,67 @@ bool kr_layout(KrPlan& p, int xrows, int experts) {
   return p.stages >= 2;
 }
 
+// Clusters of C CTAs that the GPCs hold at the same time (the kernel takes an SM per CTA whatever its shared memory); 0: none.
+template <int QT, bool FINE>
+int kr_resident(int C) {
+  if (C == 1) return rt_sm_count();
+  KrPlan p{};
+  p.C = C; p.smem = kKrSmem;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  int const most = rt_sm_count() / C;
+  kr_launch_config(cfg, at, p, unsigned(most * C), nullptr);
+  int resident = 0;
+  if (cudaOccupancyMaxActiveClusters(&resident, kq_rows_kernel<QT, FINE>, &cfg) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  return std::min(most, resident);
+}
+
 // `units`: tiles of the launch (ragged: those of a router that spreads its rows).  Plans are kept per shape.
 template <int QT, bool FINE>
 KrPlan kr_plan(int bpr, int units, int xrows, int experts) {
-  int const sms = rt_sm_count();
-  int const per_sm = std::min(64, (units + sms - 1) / sms);         // beyond that the split no longer depends on it
-  struct Key { int bpr, per, x, e, dev; bool operator<(Key const& o) const {
-    return bpr != o.bpr ? bpr < o.bpr : per != o.per ? per < o.per : x != o.x ? x < o.x : e != o.e ? e < o.e : dev < o.dev; } };
+  constexpr int kSplits[3] = {1, 2, 4};
+  units = std::min(units, 64 * rt_sm_count());                      // beyond that the split no longer depends on it
+  struct Key { int bpr, units, x, e, dev; bool operator<(Key const& o) const {
+    return bpr != o.bpr ? bpr < o.bpr : units != o.units ? units < o.units : x != o.x ? x < o.x : e != o.e ? e < o.e : dev < o.dev; } };
+  struct Slots { int n[3]; };
   static std::map<Key, KrPlan> plans;
+  static std::map<int, Slots> resident;                             // per device
   static std::mutex mu;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(mu);
-  Key const key{bpr, per_sm, xrows, experts, dev};
+  Key const key{bpr, units, xrows, experts, dev};
   auto it = plans.find(key);
   if (it != plans.end()) return it->second;
+  auto rs = resident.find(dev);
+  if (rs == resident.end()) {
+    Slots v{};
+    if (cudaFuncSetAttribute(kq_rows_kernel<QT, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKrSmem)) == cudaSuccess)
+      for (int i = 0; i < 3; ++i) v.n[i] = kr_resident<QT, FINE>(kSplits[i]);
+    else
+      (void)cudaGetLastError();
+    rs = resident.emplace(dev, v).first;
+  }
   if (plans.size() > 4096) plans.clear();
   KrPlan bestp{};
   double best = 1e30;
-  for (int C : {1, 2, 4}) {
+  for (int i = 0; i < 3; ++i) {
+    int const C = kSplits[i], slots = rs->second.n[i];
+    if (slots <= 0) continue;
     int const per_cta = (bpr + C - 1) / C, least = (per_cta + kKrWarps - 1) / kKrWarps;
     for (int passes = least; passes <= std::min(per_cta, least + 2); ++passes) {
       KrPlan p{};
-      p.C = C; p.passes = passes;
+      p.C = C; p.passes = passes; p.slots = slots;
       p.P = (per_cta + passes - 1) / passes; p.RS = kKrWarps / p.P;
       if (!kr_layout<QT>(p, xrows, experts)) continue;
       // Microseconds on 4096-deep Q4_K rows: a stage costs a latency and its warps' share of the issue slots, a pass the
-      // reload of the activations, a cluster the exchange of its sums.
-      int const rounds = (per_sm * C + p.RS - 1) / p.RS * passes;
+      // reload of the activations, a cluster the exchange of its sums.  Rounds are counted over the clusters that are resident
+      // (74 of two CTAs, but 33 of four on 148 SMs): 14336 -> 8192, Q4_K 2 rows 26.2 us as fours, 24.4 as twos, 25.8 whole, and the
+      // other way round where there are few tiles, 14336 -> 4096 15.4, 16.0, 15.9.
+      int const rounds = ((units + slots - 1) / slots + p.RS - 1) / p.RS * passes;
       double const cost = rounds * (0.4 + 0.8 * p.RS * p.P / kKrWarps) + 0.9 * passes + (C > 1 ? 1.0 : 0.0);
       if (cost < best - 1e-9) { best = cost; bestp = p; bestp.ok = 1; }
     }
-  }
-  if (bestp.ok) {
-    bestp.slots = sms / bestp.C;
-    bool fine = cudaFuncSetAttribute(kq_rows_kernel<QT, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKrSmem)) == cudaSuccess;
-    if (fine && bestp.C > 1) {                                      // clusters that the GPCs hold at the same time
-      cudaLaunchConfig_t cfg;
-      cudaLaunchAttribute at[2];
-      kr_launch_config(cfg, at, bestp, unsigned(bestp.slots * bestp.C), nullptr);
-      int resident = 0;
-      fine = cudaOccupancyMaxActiveClusters(&resident, kq_rows_kernel<QT, FINE>, &cfg) == cudaSuccess && resident > 0;
-      bestp.slots = std::min(bestp.slots, resident);
-    }
-    if (!fine) { (void)cudaGetLastError(); bestp.ok = 0; }
   }
   return plans.emplace(key, bestp).first->second;
 }

@@ -43,6 +43,18 @@ def test_q4k_sums_stay_fp32_on_deep_rows(m, n, k):
     assert kq.max_rel(out, np.concatenate([kq.vecdot_dense(blocks, x[i:i + 1], n, k, 12).reshape(1, n) for i in range(m)])) < 2e-5
 
 
+# K over clusters of two CTAs, each in two passes: many tiles of deep rows
+@pytest.mark.parametrize("qt,m,n,k", [(12, 2, 4736, 14336), (13, 5, 4736, 9216), (14, 3, 7104, 8448)])
+def test_rows_deep_and_wide(qt, m, n, k):
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=m)
+    x = synth.activations(m, k, seed=n)
+    out = qb.gguf_vecdot_rows(_cuda(blocks), _cuda(x), n, k, qt).cpu().numpy()
+    rows = np.random.default_rng(k).choice(n, 200, replace=False)
+    sub = np.ascontiguousarray(blocks.reshape(n, k // 256, -1)[rows]).reshape(200 * k // 256, -1)
+    want = x.astype(np.float64) @ kq.dequantize_f32(sub, qt).reshape(200, k).T
+    assert kq.max_rel(out[:, rows], want) < 2e-5
+
+
 @pytest.mark.parametrize("k", [2304, 4352, 13568])
 @pytest.mark.parametrize("qt", QTYPES)
 def test_error_against_64_bits(qt, k):
