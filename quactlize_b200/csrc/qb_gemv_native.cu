@@ -135,13 +135,16 @@ int enqueue_native_gemv(uint8_t const* blocks, __half const* x, float* out, int 
     //   two rows, few output rows: Q5_K n = 2400 6.6 against 7.3, n = 4800 9.3 against 9.3; a 2048-deep Q6_K 8.0 against 6.5
     //   Q2_K, the fewest bytes: 13.3 against 14.6 for two rows also at n = 14336
     //   three rows: Q5_K n = 1024 5.2 against 5.9, n = 2400 7.9 against 7.3
-    // Q4_K keeps fp32 sums from two rows up (relative error 5e-4 with the fp16 sums of the one-row kernel, 2e-7 without), at
-    // 7.0 against 5.1 us for two rows of 8192, n = 1024.
+    //   14336-deep rows: two rows Q5_K n = 2048 12.7 against 11.9, three rows Q6_K n = 1024 12.0 against 9.7 (n = 1024, 8192-deep, 7.4
+    //   against 8.1); Q2_K, two rows, n = 4096 15.3 against 17.6
+    // Q4_K keeps fp32 sums from two rows up (relative error 5e-4 with the fp16 sums of the one-row kernel, 1e-7 without), at
+    // 6.2 against 5.1 us for two rows of 8192, n = 1024.
     // Ragged launches always share: their offsets need not have been checked there, the call then has one kernel whatever the
     // type of its activations and its offsets, and sums stay fp32.  At most two rows per expert, one row per pass against it:
     // 2048-deep Q4_K, 12 rows of 32 experts, n = 8192 45.8 against 33.5, 64 rows of 128 experts, n = 1536 66.5 against 34.4; 4096-deep
     // 46.6 against 46.5, and 6 rows of 8 experts, n = 14336 39 against 45.
-    bool const one_row = !offsets && (m_rows == 1 || (qtype != 12 && bpr >= 16 && ((m_rows == 2 && (qtype == 10 || tiles <= sms)) || (m_rows == 3 && 2 * tiles <= sms))));
+    bool const few = (m_rows == 2 && (qtype == 10 || (bpr <= 32 && tiles <= sms))) || (m_rows == 3 && bpr <= 32 && 2 * tiles <= sms);
+    bool const one_row = !offsets && (m_rows == 1 || (qtype != 12 && bpr >= 16 && few));
     if (qtype == 12 && !offsets && m_rows >= 2 && m_rows <= 4 && bpr <= 16 && tiles <= 3 * sms) {
       // two to four Q4_K rows, few tiles per SM: no copy and reducing warps to start and drain (5.9 against 6.05 us at
       // n = 2400, 7.4 against 7.6 at 4800, 13.7 against 13.0 at 14336)

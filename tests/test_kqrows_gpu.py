@@ -35,12 +35,13 @@ def test_rows(qt, m, n, k):
     assert kq.max_rel(out, ref) < (4e-3 if fp16_sums else 2e-5)
 
 
-@pytest.mark.parametrize("m,n,k", [(2, 500, 8192), (3, 200, 14336), (2, 100, 4352)])
-def test_q4k_sums_stay_fp32_on_deep_rows(m, n, k):
-    blocks = synth.kquant_blocks(12, n * k // 256, seed=m)
+@pytest.mark.parametrize("qt,m,n,k", [(12, 2, 500, 8192), (12, 3, 200, 14336), (12, 2, 100, 4352),
+                                      (13, 2, 200, 14336), (14, 3, 100, 14336), (10, 3, 100, 10240), (11, 2, 60, 12288)])
+def test_sums_are_fp32_on_deep_rows(qt, m, n, k):
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=m)
     x = synth.activations(m, k, seed=n)
-    out = qb.gguf_vecdot_rows(_cuda(blocks), _cuda(x), n, k, 12).cpu().numpy()
-    assert kq.max_rel(out, np.concatenate([kq.vecdot_dense(blocks, x[i:i + 1], n, k, 12).reshape(1, n) for i in range(m)])) < 2e-5
+    out = qb.gguf_vecdot_rows(_cuda(blocks), _cuda(x), n, k, qt).cpu().numpy()
+    assert kq.max_rel(out, np.concatenate([kq.vecdot_dense(blocks, x[i:i + 1], n, k, qt).reshape(1, n) for i in range(m)])) < 2e-5
 
 
 # K over clusters of two CTAs, each in two passes: many tiles of deep rows
