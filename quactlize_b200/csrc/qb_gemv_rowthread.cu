@@ -343,9 +343,12 @@ rowthread_gemv_kernel(const __grid_constant__ CUtensorMap map_lo, const __grid_c
     mbar_init_fence();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  // No griddepcontrol.launch_dependents: the next launch may start as this one's CTAs end (the trigger their exit implies).  Triggered
+  // here, its CTAs took the SMs this launch leaves idle and waited there through the whole kernel, and launches that arrive back to
+  // back took longer: W2 gs 64, 128 experts, 64 routed rows, 1536 x 2048 19.7 us a call with the trigger here, 18.2 with it after the
+  // main loop, 18.4 without; W4 gs 128 4096 x 4096 5.1, 5.0, 4.8; the same launches from a graph 18.2-18.4 and 4.8 in all three.
   auto start_stream = [&]() {
     for (int q = 0; q < STAGES && q < ntiles; ++q) issue(q);
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   };
   if (nrows == 1) start_stream();
   for (int i = threadIdx.x; i < (nb_c + 16) * MR * TR; i += blockDim.x) part[i] = 0.f;
