@@ -14,7 +14,6 @@
 // byte-identical copies and every consumer here (GEMV and GEMM) reads Native planes.
 #include <cuda_fp16.h>
 
-#include <emmintrin.h>
 #include <sched.h>
 
 #include <algorithm>
@@ -24,6 +23,7 @@
 #include <thread>
 #include <vector>
 
+#include "qb_host_squeeze.hpp"
 #include "qb_kquant.cuh"
 
 namespace qb {
@@ -76,31 +76,7 @@ void for_rows(int64_t rows, int64_t step, int64_t bytes, Fn const& fn) {
 // ---- one superblock ---------------------------------------------------------------------------------------------------------
 //
 // The fields of consecutive code bytes belong to consecutive elements, so a run of 32 bytes shifted and masked is a run of 32
-// codes, squeezed to 4, 2 or 1 bits each with SSE2 (part of every x86-64).
-
-inline __m128i load16(uint8_t const* p) { return _mm_loadu_si128(reinterpret_cast<__m128i const*>(p)); }
-inline __m128i pair4(__m128i v, int shift) {                              // 16-bit lanes: two 4-bit codes -> one byte
-  v = _mm_srli_epi16(v, shift);
-  return _mm_or_si128(_mm_and_si128(v, _mm_set1_epi16(0x0F)), _mm_and_si128(_mm_srli_epi16(v, 4), _mm_set1_epi16(0xF0)));
-}
-inline void squeeze4(uint8_t const* src, int shift, uint8_t* dst) {       // 32 codes of 4 bits -> 16 bytes
-  _mm_storeu_si128(reinterpret_cast<__m128i*>(dst), _mm_packus_epi16(pair4(load16(src), shift), pair4(load16(src + 16), shift)));
-}
-inline __m128i quad2(__m128i v, int shift) {                              // 32-bit lanes: four 2-bit codes -> one byte
-  v = _mm_and_si128(_mm_srli_epi32(v, shift), _mm_set1_epi8(3));
-  v = _mm_or_si128(v, _mm_srli_epi32(v, 6));
-  return _mm_and_si128(_mm_or_si128(v, _mm_srli_epi32(v, 12)), _mm_set1_epi32(0xFF));
-}
-inline void squeeze2(uint8_t const* src, int shift, uint8_t* dst) {       // 32 codes of 2 bits -> 8 bytes
-  __m128i const w = _mm_packs_epi32(quad2(load16(src), shift), quad2(load16(src + 16), shift));
-  _mm_storel_epi64(reinterpret_cast<__m128i*>(dst), _mm_packus_epi16(w, w));
-}
-inline void squeeze1(uint8_t const* src, int shift, uint8_t* dst) {       // 32 codes of 1 bit -> 4 bytes
-  for (int i = 0; i < 2; ++i) {                                           // the bit moves to the top of its byte
-    uint16_t const m = uint16_t(_mm_movemask_epi8(_mm_slli_epi16(load16(src + 16 * i), 7 - shift)));
-    std::memcpy(dst + 2 * i, &m, 2);
-  }
-}
+// codes, squeezed to 4, 2 or 1 bits each (qb_host_squeeze.hpp).
 
 template <int QT>
 void planes_sb(uint8_t const* b, uint8_t* low, uint8_t* high) {           // 256 codes, offset-binary

@@ -1,5 +1,9 @@
 """The threaded, word-wide host producers against the oracle at sizes that are dealt to several threads: row counts off the
 row tile, an odd number of rows per expert, one row."""
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 import torch
@@ -28,3 +32,16 @@ def test_producers_match_the_oracle(qtype, n, k, experts):
     per = n * k // 256
     for e in range(experts):
         assert np.array_equal(units[e], np.asarray(kq.pack_units(blocks[e * per:(e + 1) * per], n, k, qtype)[0]))
+
+
+@pytest.mark.parametrize("flags", [[], ["-U__SSE2__"]])
+def test_plain_squeezer_equals_the_vector_one(tmp_path, flags):
+    """The producers build on hosts without SSE2 (the header then has the plain form only) and write the same bytes."""
+    if shutil.which("g++") is None:
+        pytest.skip("no C++ compiler")
+    here = os.path.dirname(os.path.abspath(__file__))
+    exe = tmp_path / "probe"
+    subprocess.run(["g++", "-std=c++17", "-O1", *flags, "-I", os.path.join(os.path.dirname(here), "quactlize_b200", "csrc"),
+                    os.path.join(here, "host_squeeze_probe.cpp"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
