@@ -19,7 +19,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -66,8 +66,9 @@ void for_rows(int64_t rows, int64_t step, int64_t bytes, Fn const& fn) {
   std::vector<std::thread> pool;
   int started = 1;
   try {
+    pool.reserve(nt);                                       // nothing but a thread's start can fail once one runs
     for (; started < nt; ++started) pool.emplace_back(part, started);
-  } catch (std::system_error const&) {}                     // no more threads: the rest runs here
+  } catch (std::exception const&) {}                        // no more threads or memory: the rest runs here
   part(0);
   for (int t = started; t < nt; ++t) part(t);
   for (auto& th : pool) th.join();
