@@ -128,7 +128,7 @@ def lib():
 
 
 class _Native:
-    """The CPython binding of the device-tensor calls (_native.so), loaded and bound to `lib()` on first use; afterwards
+    """The CPython binding of the device-tensor calls (build.native_path()), loaded and bound to `lib()` on first use; afterwards
     its functions are plain attributes of this object."""
 
     def __getattr__(self, name):
@@ -136,8 +136,8 @@ class _Native:
             raise AttributeError(name)
         import importlib.machinery
         import importlib.util
-        import torch  # noqa: F401  -- its libraries have to be loaded first
-        path = os.path.join(_HERE, "_native.so")
+        from .build import native_path
+        path = native_path()                 # imports torch, whose libraries have to be loaded first
         if not os.path.exists(path):
             raise ImportError(f"{path} is not built. Build it with:  python -m quactlize_b200.build")
         h = lib()

@@ -2,8 +2,10 @@
 
     python -m quactlize_b200.build [-v] [--force]
 
-and, beside it, quactlize_b200/_native.so: the CPython binding of the device-tensor calls (csrc/qb_torch.cpp, host code only,
-compiled with g++ against torch's headers and linked to torch's libraries).
+and, beside it, quactlize_b200/_native.<python ABI>.torch-<version>.so: the CPython binding of the device-tensor calls
+(csrc/qb_torch.cpp, host code only, compiled with g++ against torch's headers and linked to torch's libraries).  The library does not
+depend on it: it is linked first, and where torch is not installed it is all that is built (`python quactlize_b200/build.py` needs
+the standard library only).
 
     python -m quactlize_b200.build --variant NAME --define MACRO[=VALUE] [--define ...]
 
@@ -36,15 +38,28 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
 
 
 NATIVE_SRC = os.path.join(CSRC, "qb_torch.cpp")
-NATIVE = os.path.join(HERE, "_native.so")
 
 
-def build_native(verbose: bool = False, force: bool = False) -> str:
-    """The CPython binding; rebuilt when its source or the C-ABI header changed."""
-    header = os.path.join(os.path.dirname(HERE), "include", "quactlize_b200.h")
-    newest = max(os.path.getmtime(NATIVE_SRC), os.path.getmtime(header))
-    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest:
-        return NATIVE
+def native_path() -> str:
+    """Where the binding for this interpreter and this torch lies.  It is compiled against the C++ ABI of the one and the C ABI of
+    the other, so both are in its name: after an upgrade of either it is a file that has to be built."""
+    import sysconfig
+
+    import torch
+    return os.path.join(HERE, f"_native.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
+
+
+def build_native(verbose: bool = False, force: bool = False):
+    """The CPython binding; rebuilt when its source, the C-ABI header or this file changed.  None where there is no torch."""
+    import importlib.util
+    if importlib.util.find_spec("torch") is None:
+        print("torch is not installed: the CPython binding is not built", flush=True)
+        return None
+    path = native_path()
+    newest = max(os.path.getmtime(f) for f in (NATIVE_SRC, os.path.join(os.path.dirname(HERE), "include", "quactlize_b200.h"),
+                                               os.path.abspath(__file__)))
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= newest:
+        return path
     import sysconfig
 
     import torch
@@ -54,14 +69,14 @@ def build_native(verbose: bool = False, force: bool = False) -> str:
                 sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{i}" for i in includes], NATIVE_SRC,
-           "-o", NATIVE, f"-L{libdir}", f"-Wl,-rpath,{libdir}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch",
+           "-o", path, f"-L{libdir}", f"-Wl,-rpath,{libdir}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch",
            "-lc10_cuda", "-lc10"]
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
-    return NATIVE
+    return path
 
 
 def sources():
@@ -99,9 +114,9 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
     with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)) + 1)) as ex:
         native = ex.submit(build_native, verbose, force)
         list(ex.map(run, jobs))
+        if jobs or not os.path.exists(LIB):
+            run([NVCC, "-shared", "-o", LIB, *objs, "-cudart", "shared"])
         native.result()
-    if jobs or not os.path.exists(LIB):
-        run([NVCC, "-shared", "-o", LIB, *objs, "-cudart", "shared"])
     return LIB
 
 
