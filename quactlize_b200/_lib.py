@@ -4,6 +4,8 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # QUACTLIZE_B200_LIB selects another build of the same library (as QUACTLIZE_PPU_LIB does for the reference loader)
@@ -129,24 +131,40 @@ def lib():
 
 class _Native:
     """The CPython binding of the device-tensor calls (build.native_path()), loaded and bound to `lib()` on first use; afterwards
-    its functions are plain attributes of this object."""
+    its functions are plain attributes of this object.  Where it is not built or does not load, every function returns None -- the
+    answer for a call it does not serve -- after one warning, and the calls take the Python path above the same library."""
 
-    def __getattr__(self, name):
-        if name.startswith("__"):
-            raise AttributeError(name)
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._absent = False
+
+    def _load(self, h):
         import importlib.machinery
         import importlib.util
         from .build import native_path
         path = native_path()                 # imports torch, whose libraries have to be loaded first
         if not os.path.exists(path):
             raise ImportError(f"{path} is not built. Build it with:  python -m quactlize_b200.build")
-        h = lib()
         full = __package__ + "._native"
         loader = importlib.machinery.ExtensionFileLoader(full, path)
         m = importlib.util.module_from_spec(importlib.util.spec_from_file_location(full, path, loader=loader))
         loader.exec_module(m)
         m.bind({n: C.cast(getattr(h, n), C.c_void_p).value for n in m.entries()})
-        self.__dict__.update({k: v for k, v in vars(m).items() if not k.startswith("__")})
+        return {k: v for k, v in vars(m).items() if not k.startswith("__")}
+
+    def __getattr__(self, name):
+        if name.startswith("_"):
+            raise AttributeError(name)
+        h = lib()                            # a missing library raises, as everywhere
+        with self._lock:
+            if name not in self.__dict__ and not self._absent:
+                try:
+                    self.__dict__.update(self._load(h))
+                except ImportError as e:
+                    self._absent = True
+                    warnings.warn(f"the native call path is not available, calls take about 15 us longer: {e}", RuntimeWarning, stacklevel=3)
+            if self._absent:
+                self.__dict__[name] = lambda *args: None
         return self.__dict__[name]
 
 
