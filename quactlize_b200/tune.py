@@ -11,6 +11,8 @@ Follows the behaviour of the reference's tools/tune.py (policy statements :28-41
     maps to another bucket misses and takes the compiled default; a winner is never extended beyond its evidence;
   * a sweep that does not separate its candidates (the best two medians closer than the observed spread) records NO
     winner -- an absent tactic gets the default, a wrong one does not get noticed;
+  * the library's own choice (no name) runs in every device sweep: it has forms that no name forces (K cut over a cluster), and a
+    tactic is recorded only where it is separated from that choice too.  Where the choice is the fastest nothing is recorded;
   * every table carries its provenance: the library file's hash, the hash of the inventory it was chosen from, the
     device, the workload, repetitions.
 
@@ -36,6 +38,7 @@ CACHE_SCHEMA = "quactlize-ppu-tactic-cache-v1"
 BUCKET_POLICY = "last-positive-power-of-two(raw-total-tokens);store-only-profiled-buckets;v1"
 ROUTE_SCHEMA = "route+normalized-op+qtype+n+k+group-size+m-bucket+experts+top-k;v2"
 ROUTES = ("dense_fully_quantized", "grouped_fully_quantized")
+DEFAULT = ""                                               # the name that leaves the form to the library
 _FNV_OFFSET, _FNV_PRIME = 14695981039346656037, 1099511628211
 
 # model name -> (FFN projections [(op, n, k)], experts, top_k); shapes of the benchmark configurations
@@ -97,14 +100,15 @@ def m_bucket(m: int) -> int:
 
 
 def measured_buckets(by_m: Dict[int, str]) -> List[dict]:
-    """Resolved measurements -> exact bucket winners.  Two measurements that fall in one bucket must agree."""
+    """Resolved measurements -> exact bucket winners.  Two measurements that fall in one bucket must agree.  A bucket that the
+    library's own choice wins is left out: its absence means just that."""
     out: Dict[int, dict] = {}
     for m in sorted(by_m):
         b = m_bucket(m)
         if b in out and out[b]["config"] != by_m[m]:
             raise ValueError(f"M={out[b]['measured_m']} and M={m} map to bucket {b} but disagree")
         out[b] = {"m_bucket": b, "measured_m": m, "config": by_m[m]}
-    return [out[b] for b in sorted(out)]
+    return [out[b] for b in sorted(out) if out[b]["config"] != DEFAULT]
 
 
 def pick_winner(samples: Dict[str, Sequence[float]]) -> Tuple[Optional[str], str]:
@@ -120,7 +124,7 @@ def pick_winner(samples: Dict[str, Sequence[float]]) -> Tuple[Optional[str], str
     best, second = med[0], med[1]
     if max(samples[best[1]]) < second[0]:
         return best[1], "separated"
-    return None, f"unresolved: {best[1]} {best[0]:.2f} us vs {second[1]} {second[0]:.2f} us overlap"
+    return None, f"unresolved: {best[1] or 'default'} {best[0]:.2f} us vs {second[1] or 'default'} {second[0]:.2f} us overlap"
 
 
 def valid_candidates(lib, route: str, inventory: List[dict], m: int, n: int, k: int, gs: int, qtype: int, experts: int, topk: int):
@@ -192,14 +196,16 @@ def device_timer(lib, route: str, n: int, k: int, qtype: int, experts: int, topk
 
 
 def tune(lib, model: str, route: str, qtype: int, ms: Sequence[int], reps: int,
-         timer_for: Optional[Callable[[int, int], Callable[[int, str], float]]] = None) -> dict:
+         timer_for: Optional[Callable[[int, int], Callable[[int, str], float]]] = None, with_default: Optional[bool] = None) -> dict:
     """Sweep every distinct (n, k) of the model over `ms`; returns the table (resolved winners only, plus the raw
-    medians and the notes of unresolved sweeps).  `timer_for(n, k)` supplies the timer (the device one by default)."""
+    medians and the notes of unresolved sweeps).  `timer_for(n, k)` supplies the timer (the device one by default);
+    `with_default` times the library's own choice among the candidates (by default: with the device timer)."""
     if reps < 2:
         raise ValueError("reps must be at least 2: one pass cannot separate candidates")
     if route not in ROUTES:
         raise ValueError(f"route must be one of {ROUTES}")
     cfg = MODELS[model]
+    with_default = timer_for is None if with_default is None else with_default
     grouped = route == "grouped_fully_quantized"
     if grouped and not cfg["experts"]:
         raise ValueError(f"{model} has no experts; use the dense route")
@@ -213,12 +219,13 @@ def tune(lib, model: str, route: str, qtype: int, ms: Sequence[int], reps: int,
         by_m, raw = {}, []
         for m in ms:
             cands = valid_candidates(lib, route, inventory, m, n, k, gs, qtype, cfg["experts"], cfg["topk"])
+            cands += [DEFAULT] if with_default and cands else []
             samples: Dict[str, List[float]] = {c: [] for c in cands}
             for _ in range(reps):                          # interleave the candidates across repetitions
                 for c in cands:
                     samples[c].append(timer(m, c))
             winner, note = pick_winner(samples)
-            raw.append({"m": m, "note": note, "median_us": {c: round(statistics.median(v), 3) for c, v in samples.items() if v}})
+            raw.append({"m": m, "note": note, "median_us": {c or "default": round(statistics.median(v), 3) for c, v in samples.items() if v}})
             if winner is not None:
                 by_m[m] = winner
         shapes.append({"n": n, "k": k, "buckets": measured_buckets(by_m), "sweeps": raw})

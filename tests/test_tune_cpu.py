@@ -74,3 +74,18 @@ def test_grouped_route_uses_the_grouped_predicate():
                       timer_for=lambda n, k: (lambda m, t: seen.append((m, t)) or {"128x128x64:tcgen05": 10.0, "256x256x64:tcgen05": 20.0}.get(t, 15.0)))
     assert {t for _, t in seen} == {"256x256x64:tcgen05", "128x128x64:tcgen05", "128x128x64:tcgen05:splitk"}
     assert all(s["buckets"][0]["config"] == "128x128x64:tcgen05" for s in table["shapes"])
+
+
+def test_a_tactic_has_to_beat_the_librarys_own_choice():
+    """The library's choice has forms that no name forces: where it is the fastest, or not separated, nothing is pinned."""
+    lib = _lib.lib()
+    us = {16: {"": 12.0, "128x128x64:tcgen05": 38.0, "256x256x64:tcgen05": 60.0},       # the choice wins
+          64: {"": 30.0, "128x128x64:tcgen05": 30.0, "256x256x64:tcgen05": 60.0},       # it is one of the tactics
+          1024: {"": 50.0, "128x128x64:tcgen05": 70.0, "256x256x64:tcgen05": 40.0}}     # a tactic wins
+    table = tune.tune(lib, "llama3-8b", "dense_fully_quantized", 12, [16, 64, 1024], reps=2, timer_for=lambda n, k: (lambda m, t: us[m][t]),
+                      with_default=True)
+    for s in table["shapes"]:
+        assert s["buckets"] == [{"m_bucket": 1024, "measured_m": 1024, "config": "256x256x64:tcgen05"}]
+        assert s["sweeps"][0]["median_us"]["default"] == 12.0 and s["sweeps"][1]["note"].startswith("unresolved")
+    with pytest.raises(ValueError):
+        tune.measured_buckets({64: "", 100: "a"})
