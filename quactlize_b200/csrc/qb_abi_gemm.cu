@@ -22,7 +22,8 @@ using namespace qb;
 
 namespace {
 // Two tensor-core tactics are compiled (CTA tile 256 x 256 and 128 x 128, K stage 64); a null or empty name lets the launcher
-// choose by rows per expert, a known name forces that tile, an unknown name is declined with a message and the default runs.
+// choose (gemm_form in qb_gemm.cu: also forms that no name forces, with K cut over a cluster), a known name forces that tile with K
+// whole, an unknown name is declined with a message and the default runs.
 constexpr char const* kTensorConfig = "256x256x64:tcgen05";
 constexpr char const* kTensorConfigSmall = "128x128x64:tcgen05";
 // grouped only: the decode tactic -- 128 x 128 tiles with two-deep rings (several CTAs per SM) and K split over gridDim.z

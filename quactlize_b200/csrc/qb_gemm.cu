@@ -1210,16 +1210,24 @@ bool tma_make_map(CUtensorMap* m, CUtensorMapDataType dt, int rank, void const* 
 long long gemm_swap_launches() { return g_swap_launches.load(std::memory_order_relaxed); }
 
 // Which form a problem takes: the 256 x 256 tile (one CTA per SM), or 128 x 128 tiles, on four-deep rings where an SM gets one
-// CTA (m = 17, n = 4096 39.3 against 41.6 us) and on two-deep ones, two CTAs per SM, where there are more; for a dense problem
+// CTA (m = 17, n = 4096, k = 2048 27.4 against 28.4 us) and on two-deep ones, two CTAs per SM, where there are more; for a dense problem
 // with K cut over a cluster of 2, 4 or 8 CTAs that add their slices through shared memory.  Microseconds, from
 // 64-k stages: a wave of 256 x 256 tiles 6 + 0.9 a stage whatever its rows; of 128 x 128 tiles 0.6 a stage with one CTA on an
 // SM and 0.78 with two, and 5 for the pipeline's fill, drain and launch (7 with the exchange of a cluster, 8 with eight CTAs).
 // Measured on 4096-deep int4, us: m = 17, n = 1024 37.7 -> 12.7 (8 slices); m = 256, n = 4096 59.9 -> 23.0 (4); m = 190,
-// n = 14336 77 -> 54.6 (none); m = 333, n = 14336 62.6 as 256 x 256 tiles, 85-95 as the others.  Ragged problems are not cut
-// in K: a row's bits then do not depend on which other rows, experts or ranks share the launch.  Nor are dense ones of up to
-// 2048 k, where the cut gives least (m = 190, n = k = 1024: 10.7 against 14.7): there every form of the kernel, and an expert
-// alone against its rows of a ragged launch, agree to the last bit.  The tile counts of ragged problems are an estimate (half
-// a tile is padding per expert, one tile at least): 8 experts, 1200 rows, n = 8192 225 -> 118.
+// n = 14336 77 -> 54.6 (none); m = 333, n = 14336 62.6 as 256 x 256 tiles, 85-95 as the others.
+// The constants are those of int4 with groups of 64; more groups and a second plane cost a stage 10 to 50 % more in either tile, so one
+// rule serves all widths: on 22 problems each of int4 gs 32, int2 gs 16, 2+1, 4+1 and 4+2 bits gs 16 / 32 and int1 (m 17 to 1000, k 1024 to
+// 8192, 8 and 16 experts with 100 to 8192 rows) the form taken is the fastest or within 7 % of it where K may be cut or is whole
+// in either, and 9 to 13 % behind 256 x 256 tiles on ragged problems of under 100 rows an expert (8 experts, 600 rows, n = 8192, int4 124
+// against 111).  Against 256 x 256 tiles from 192 rows up, none is more than 3 % slower (4+2 bits, m = 1000, n = 4096, k = 2048 51.0 against
+// 50.0), the others up to 4.8 times faster.
+// Ragged problems are not cut in K: a row's bits then do not depend on which other rows, experts or ranks share the launch.  Nor
+// are dense ones of up to 2048 k.  That line is not one of speed (m = 64, n = 4096, k = 2048 27.8 against 12.5 with four slices) but of what
+// callers rely on: up to there every form of the kernel agrees to the last bit, and an expert alone with its rows of a ragged launch.
+// Beyond it a dense call without a tactic's name may be cut, and its last bits then depend on m and n; a named tactic is never cut.
+// The tile counts of ragged problems are an estimate (half a tile is padding per expert, one tile at least): 8 experts, 1200 rows,
+// n = 8192 225 -> 118.
 struct GemmForm { bool big, shallow; int splits; };
 GemmForm gemm_form(GemmDesc const& d) {
   double const stages = d.k / kTK;

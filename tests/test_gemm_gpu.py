@@ -267,3 +267,43 @@ def test_k_cut_over_a_cluster_two_planes(qt):
     a = synth.activations(m, k, seed=4)
     out = qb.gguf_dense_fully_quantized(_cuda(a), low, high, units, qt)
     _check(out, a.astype(np.float64) @ kq.dequantize_f32(blocks, qt).reshape(n, k).T.astype(np.float64))
+
+
+# What holds beyond 2048 k, where a dense call without a name may have K cut: a named tactic, and a ragged launch, are never cut, so
+# a row's bits do not depend on the rows beside it; the unnamed call repeats itself.
+def test_bits_of_a_row_beyond_2048_k():
+    n, k, qt, big = 256, 4352, 12, 300
+    L = _lib.lib()
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=3)
+    low, high, units = (t.to(DEV) for t in qb.gguf_prepare_fully_quantized_dense(torch.from_numpy(blocks), n, k, qt))
+    a = _cuda(synth.activations(big, k, seed=4))
+
+    def call(m, name):
+        out = torch.empty((m, n), dtype=torch.float16, device=DEV)
+        need = L.quactlize_ppu_dense_fully_quantized_workspace_bytes_v1(m, n, k, qt)
+        ws = torch.empty(max(need, 1), dtype=torch.uint8, device=DEV)
+        rc = L.quactlize_ppu_dense_fully_quantized_dev_v2(a.data_ptr(), low.data_ptr(), None, units.data_ptr(), out.data_ptr(), m, n, k, qt,
+                                                          ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream, name)
+        assert rc == 0
+        return out
+
+    whole = call(big, b"256x256x64:tcgen05")
+    for m in (1, 17, 129, 300):
+        for name in (b"256x256x64:tcgen05", b"128x128x64:tcgen05"):
+            assert torch.equal(call(m, name), whole[:m]), (m, name)
+        unnamed = call(m, b"")
+        assert torch.equal(unnamed, call(m, b""))
+        _check(unnamed, whole[:m].double().cpu().numpy())
+
+
+def test_an_expert_alone_beyond_2048_k():
+    n, k, counts = 256, 4352, [3, 0, 140, 17]
+    low, scale, zp = (_cuda(t) for t in synth.group_planes(4, n, k, 4, 64, seed=5))
+    a = _cuda(synth.activations(sum(counts), k, seed=6))
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    ragged = qb.gemm_plane(a, low, None, scale, zp, 4, 0, 64, row_offsets=_cuda(off))
+    for e in range(4):
+        rows = slice(off[e], off[e + 1])
+        if counts[e]:                                                        # split_k = 1: one slice, K whole
+            solo = qb.gemm_plane(a[rows], low[e:e + 1], None, scale[e:e + 1], zp[e:e + 1], 4, 0, 64, split_k=1)
+            assert torch.equal(solo, ragged[rows]), e
