@@ -1,27 +1,25 @@
-// Dense raw GGUF Q4_K GEMV for 2..8 activation rows: the tensor-core arithmetic of the small-batch kernel on the copy
-// structure of the single-row kernel, so that eight rows cost what one row costs -- the weights are streamed once,
-// in large contiguous pieces, and the kernel stays bound by that stream.
+// Dense raw GGUF Q4_K GEMV for two to four activation rows of at most 4096 and few output rows per SM: the tensor-core arithmetic
+// on the copy structure of the single-row kernel.  The several-row kernel (qb_gemv_kqrows.cu) takes everything else; here there are
+// no copy and reducing warps to start and drain (2 rows, 4096 -> 2400: 5.2 against 6.0 us; 4 rows -> 7000 7.4 against 8.6; the
+// launch policy has the line).
 //
 //   out[t, r] = sum_b sum_g ( d_rb*sc_rbg * sum_j q_rbgj x[t, 256b+32g+j]  -  dmin_rb*mn_rbg * sum_j x[t, 256b+32g+j] )
 //
 // Same contract as the M > 1 arm of the reference's vecdot_rows_kernel (quactlize/include/gguf_vecdot.hpp:604-760).
 //
 // Work split.  A CTA (16 warps, one per SM) owns a run of consecutive output rows (dealt over the grid in units of eight)
-// and walks it in TILES of 16 rows.  K is covered in PASSES of at most 16 superblocks; in a pass warp w owns superblock w
-// of every row of the tile.  A stage of the shared-memory ring is one (pass, tile): 16 bulk copies, one per row, each
-// the row's contiguous run of this pass's superblocks (2.3 KB at K = 4096), completing on one mbarrier; rows are padded
-// apart so the fragment loads of a warp fall on 32 different banks.  Every wait is bounded.
+// and walks it in TILES of 16 rows; warp w owns superblock w of every row of the tile.  A stage of the shared-memory ring is
+// one tile: 16 bulk copies, one per row (2.3 KB at K = 4096), completing on one mbarrier; rows are padded apart so the fragment
+// loads of a warp fall on 32 different banks.  Every wait is bounded.
 //
 // Arithmetic.  mma.sync.m16n8k16: the packed nibbles ARE the A fragments -- (word & 0x000F000F) read as fp16 is two codes
-// * 2^-24, (word & 0x00F000F0) two codes * 2^-20 of the neighbouring group -- and the activations of up to eight rows,
-// pre-scaled by a power of two per (row, superblock), are the B fragments, held in REGISTERS for the whole pass (32 per
-// lane).  The fp32 products of a 32-code group are scaled by d*sc and accumulated; lane t of a quad unpacks the 6-bit
+// * 2^-24, (word & 0x00F000F0) two codes * 2^-20 of the neighbouring group -- and the activations, pre-scaled by a power of two
+// per (row, superblock), are the B fragments, held in REGISTERS throughout (32 per lane).  The fp32 products of a 32-code group are scaled by d*sc and accumulated; lane t of a quad unpacks the 6-bit
 // sub-scales and sub-mins of groups 2t, 2t+1 of its two rows, the quad exchanges d*sc through 512 bytes of shared memory,
 // and the sub-mins go through one more MMA (m16n8k8) against the per-group sums of x, split in two fp16 halves so the
-// fp32 sums are kept.  A warp keeps its K-slice of every tile of the CTA in its own area of shared memory across the
-// passes (registers go to the B fragments); the slices of a row are added in warp order at the end, so results do not
-// depend on timing.  The activations of the first pass are requested before the first weight copy: a load requested
-// behind the ring's copies is served after them.
+// fp32 sums are kept.  A warp keeps its K-slice of every tile of the CTA in its own area of shared memory; the slices of a row
+// are added in warp order at the end, so results do not depend on timing.  The activations are requested before the first weight
+// copy: a load requested behind the ring's copies is served after them.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -41,14 +39,14 @@ namespace {
 constexpr int kTileRows = 16;
 constexpr int kRWarps = 16;
 constexpr int kMaxTiles = 7;             // tiles per CTA (at most 112 rows): bounds the shared memory of the K-slices
-constexpr int kCols = 8;                 // the n of the MMA = activation rows per launch
+constexpr int kCols = 8;                 // the n of the MMA
+constexpr int kMaxRows = 4;              // activation rows per launch: from five the several-row kernel is as fast
 
 struct RowsArgs {
   uint8_t const* blocks;
   __half const* x;
   float* out;
-  int n, bpr, m;                         // output rows, superblocks per row, activation rows (1..8)
-  int passes, nbp;                       // K passes; superblocks per pass (<= 16)
+  int n, bpr, m;                         // output rows, superblocks per row (<= 16), activation rows
   int pitch, stages;                     // bytes between the rows of a staged tile; ring depth
   int units_q, units_r;                  // CTA c owns units_q (+1 if c < units_r) units of eight rows
   unsigned int* status;
@@ -62,11 +60,6 @@ __device__ __forceinline__ uint2 r_lds64(uint32_t a) {
 __device__ __forceinline__ uint4 r_lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ float2 r_ldsf2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
   return v;
 }
 __device__ __forceinline__ void r_stsf2(uint32_t a, float x, float y) {
@@ -130,7 +123,6 @@ __global__ void __launch_bounds__(kRWarps * 32, 1) q4k_rows_kernel(RowsArgs a) {
   int const row0 = u0 * 8, nrows = min(a.n, row0 + nu * 8) - row0;
   if (nrows <= 0) return;                                                 // uniform, before any barrier
   int const ntiles = (nrows + kTileRows - 1) / kTileRows;
-  int const total = ntiles * a.passes;                                    // stages this CTA consumes
   // ---- shared memory: ring | barriers | d*sc exchange ---------------------------------------------------------------------
   uint32_t const s0 = smem_u32(smem);
   uint32_t const stage_bytes = uint32_t(kTileRows) * uint32_t(a.pitch);
@@ -152,32 +144,30 @@ __global__ void __launch_bounds__(kRWarps * 32, 1) q4k_rows_kernel(RowsArgs a) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  // stage q = (pass q / ntiles, tile q % ntiles); warp 0 issues it: lane 0 arms the barrier, lane r copies row r
-  auto issue = [&](int p, int tl, int s) {
-    int const rows_t = min(kTileRows, nrows - tl * kTileRows), nb = min(a.nbp, a.bpr - p * a.nbp);
-    unsigned const bytes = unsigned(nb) * 144u;
+  // a stage is a tile; warp 0 issues it: lane 0 arms the barrier, lane r copies row r
+  auto issue = [&](int tl, int s) {
+    int const rows_t = min(kTileRows, nrows - tl * kTileRows);
+    unsigned const bytes = unsigned(row_stride);
     uint32_t const bar = full32 + 8u * s;
     if (lane == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(unsigned(rows_t) * bytes) : "memory");
     __syncwarp();
     if (lane < rows_t) {
-      uint8_t const* src = a.blocks + size_t(row0 + tl * kTileRows + lane) * row_stride + size_t(p) * a.nbp * 144;
+      uint8_t const* src = a.blocks + size_t(row0 + tl * kTileRows + lane) * row_stride;
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                    ::"r"(ring32 + uint32_t(s) * stage_bytes + uint32_t(lane) * uint32_t(a.pitch)), "l"(src), "r"(bytes), "r"(bar) : "memory");
     }
   };
-  int ip = 0, itl = 0;                                                    // (pass, tile) of the next stage to request
+  int itl = 0;                                                            // the next tile to request
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   uint16_t const* xg = reinterpret_cast<uint16_t const*>(a.x) + size_t(g) * (size_t(a.bpr) * 256);   // activation row g = MMA column g
   bool const col_live = g < a.m;
   bool dead = false;
-  int q = 0, s = 0, ps = 0;                                                // stage counter; its ring slot; the previous slot
+  int s = 0, ps = 0;                                                       // ring slot of the tile; the previous slot
   unsigned par = 0u, ppar = 0u;                                            // ... and their phase parities
-  for (int p = 0; p < a.passes && !dead; ++p) {
-    int const nb = min(a.nbp, a.bpr - p * a.nbp);
-    bool const active = warp < nb;                                         // this warp has a superblock in this pass
-    int const blk = p * a.nbp + warp;
+  {
+    bool const active = warp < a.bpr;                                      // this warp has a superblock
     // ---- B fragments of this warp's superblock: eight columns (activation rows), pre-scaled by a power of two per
     // (column, superblock); group sums for the sub-min term ------------------------------------------------------------
     uint32_t xb[4][8];
@@ -189,19 +179,14 @@ __global__ void __launch_bounds__(kRWarps * 32, 1) q4k_rows_kernel(RowsArgs a) {
       uint4 raw[8];
       float mx = 0.f;
       bool const ld = active && col_live;
-      uint4 const* xp = reinterpret_cast<uint4 const*>(xg + size_t(blk) * 256);
+      uint4 const* xp = reinterpret_cast<uint4 const*>(xg + size_t(warp) * 256);
       if (ld) {
 #pragma unroll
         for (int gr = 0; gr < 8; ++gr) raw[gr] = r_ldg128(xp + gr * 4 + t);   // elements 8t..8t+7 of group gr
       }
-      if (p == 0) {
-        __syncthreads();                                                   // every warp's loads are requested
-        if (warp == 0)
-          for (int qq = 0; qq < S && qq < total; ++qq) {
-            issue(ip, itl, qq);
-            if (++itl == ntiles) { itl = 0; ++ip; }
-          }
-      }
+      __syncthreads();                                                     // every warp's loads are requested
+      if (warp == 0)
+        for (; itl < S && itl < ntiles; ++itl) issue(itl, itl);
       // group sums for the sub-min term, from the registers: this lane has eight elements of each of the eight groups;
       // a two-step exchange inside the quad leaves lane t with the whole sums of groups 2t and 2t+1
       float ps[8];
@@ -263,17 +248,16 @@ __global__ void __launch_bounds__(kRWarps * 32, 1) q4k_rows_kernel(RowsArgs a) {
       f0 = __shfl_sync(0xffffffffu, fm, 8 * t);
       f1 = __shfl_sync(0xffffffffu, fm, 8 * t + 4);
     }
-    // ---- the tiles of this pass ---------------------------------------------------------------------------------------
+    // ---- the tiles ---------------------------------------------------------------------------------------
     // The body appears once (unrolled over the tiles it would not fit the instruction cache); the accumulator set of the
     // tile is picked by a switch at the end, so the sets stay in registers.
 #pragma unroll 1
     for (int tl = 0; tl < ntiles; ++tl) {
       if (dead) break;                                                     // uniform for the warp
-      if (warp == 0 && q >= 1 && ip < a.passes) {                          // refill the slot the CTA finished one stage ago
+      if (warp == 0 && tl >= 1 && itl < ntiles) {                          // refill the slot the CTA finished one stage ago
         if (!r_wait(empty32 + 8u * ps, ppar, a.status)) dead = true;
         else {
-          issue(ip, itl, ps);
-          if (++itl == ntiles) { itl = 0; ++ip; }
+          issue(itl++, ps);
         }
       }
       dead = __shfl_sync(0xffffffffu, int(dead), 0) != 0;
@@ -329,20 +313,13 @@ __global__ void __launch_bounds__(kRWarps * 32, 1) q4k_rows_kernel(RowsArgs a) {
         r_mma8(cm, am0, am1, sx_lo);
         float const r0 = fmaf(f0, bacc[0], -ddl.y * cm[0]), r1 = fmaf(f1, bacc[1], -ddl.y * cm[1]);
         float const r2 = fmaf(f0, bacc[2], -ddh.y * cm[2]), r3 = fmaf(f1, bacc[3], -ddh.y * cm[3]);
-        // this warp's K-slice of the tile: kept in shared memory across the passes (its own area: no other warp touches it)
+        // this warp's K-slice of the tile, in its own area of shared memory
         uint32_t const ra = red32 + uint32_t(((warp * ntiles + tl) * kTileRows + g) * kCols + 2 * t) * 4u;
-        if (p == 0) {
-          r_stsf2(ra, r0, r1);
-          r_stsf2(ra + 8u * kCols * 4u, r2, r3);
-        } else {
-          float2 const o0 = r_ldsf2(ra), o1 = r_ldsf2(ra + 8u * kCols * 4u);
-          r_stsf2(ra, o0.x + r0, o0.y + r1);
-          r_stsf2(ra + 8u * kCols * 4u, o1.x + r2, o1.y + r3);
-        }
+        r_stsf2(ra, r0, r1);
+        r_stsf2(ra + 8u * kCols * 4u, r2, r3);
       }
       __syncwarp();                                                        // every lane's reads of the stage are done
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty32 + 8u * s) : "memory");
-      ++q;
       ps = s; ppar = par;
       if (++s == S) { s = 0; par ^= 1u; }
     }
@@ -360,19 +337,19 @@ __global__ void __launch_bounds__(kRWarps * 32, 1) q4k_rows_kernel(RowsArgs a) {
     int const col = o / (ntiles * kTileRows), rr = o % (ntiles * kTileRows);  // consecutive threads -> consecutive output rows
     if (rr >= nrows || col >= a.m) continue;
     float sum = 0.f;
-    for (int w = 0; w < a.nbp; ++w) sum += red[(size_t(w) * ntiles * kTileRows + rr) * kCols + col];   // warps >= nbp never had a superblock
+    for (int w = 0; w < a.bpr; ++w) sum += red[(size_t(w) * ntiles * kTileRows + rr) * kCols + col];   // the other warps had no superblock
     a.out[size_t(col) * a.n + row0 + rr] = sum;
   }
 }
 
-struct RowsPlan { int gx, passes, nbp, pitch, stages, units_q, units_r, ok; size_t smem; };
+struct RowsPlan { int gx, pitch, stages, units_q, units_r, ok; size_t smem; };
 
 }  // namespace
 
 // Enqueue; false when the shape is outside this kernel's envelope (the caller then uses another kernel).
 bool enqueue_q4k_rows(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, unsigned int* status,
                       cudaStream_t stream) {
-  if (n <= 0 || bpr <= 0 || rows <= 0 || rows > kCols || !status) return false;
+  if (n <= 0 || bpr <= 0 || bpr > kRWarps || rows <= 0 || rows > kMaxRows || !status) return false;
   if ((reinterpret_cast<uintptr_t>(blocks) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return false;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); return false; }
@@ -386,11 +363,9 @@ bool enqueue_q4k_rows(uint8_t const* blocks, __half const* x, float* out, int n,
     auto it = plans.find(key);
     if (it == plans.end()) {
       int const sms = rt_sm_count();
-      p.passes = (bpr + kRWarps - 1) / kRWarps;
-      p.nbp = (bpr + p.passes - 1) / p.passes;
       // rows of a staged tile sit pitch bytes apart with (pitch / 4) % 32 == 8: an 8-byte fragment load is served half a
       // warp at a time (rows g = 0..3 or 4..7, four lanes of 8 bytes each), and those four rows then tile the 32 banks
-      int const words = p.nbp * 36;
+      int const words = bpr * 36;
       p.pitch = (words + ((8 - words % 32) + 32) % 32) * 4;
       int const units = (n + 7) / 8;
       p.gx = std::max(std::min(sms, units), (units + (kMaxTiles * 2) - 1) / (kMaxTiles * 2));
@@ -413,7 +388,7 @@ bool enqueue_q4k_rows(uint8_t const* blocks, __half const* x, float* out, int n,
   if (!p.ok) return false;
   RowsArgs a{};
   a.blocks = blocks; a.x = x; a.out = out; a.n = n; a.bpr = bpr; a.m = rows;
-  a.passes = p.passes; a.nbp = p.nbp; a.pitch = p.pitch; a.stages = p.stages; a.units_q = p.units_q; a.units_r = p.units_r;
+  a.pitch = p.pitch; a.stages = p.stages; a.units_q = p.units_q; a.units_r = p.units_r;
   a.status = status;
   static bool const no_pdl = std::getenv("QUACTLIZE_B200_NO_PDL") != nullptr;
   cudaLaunchConfig_t cfg{};

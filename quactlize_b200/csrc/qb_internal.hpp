@@ -16,7 +16,7 @@ bool enqueue_q4k_gemv1(uint8_t const* blocks, __half const* x, float* out, int n
 bool enqueue_q4k_gemv1_dual(uint8_t const* blocks1, int n1, uint8_t const* blocks2, int n2, __half const* x, float* out1, float* out2,
                             int bpr, unsigned int* status, cudaStream_t stream);   // two matrices, one activation row, one launch
 bool enqueue_q4k_rows(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, unsigned int* status,
-                      cudaStream_t stream);                 // dense, 1..8 rows, tensor cores on the single-row kernel's copy structure
+                      cudaStream_t stream);                 // dense, up to 4 rows of at most 4096, tensor cores on the single-row kernel's copy structure
 bool enqueue_kquant_gemv1(uint8_t const* blocks, __half const* x, float* out, int n, int bpr, int rows, int qtype, unsigned int* status,
                           cudaStream_t stream);             // Q2_K/Q3_K/Q5_K/Q6_K, dense, one row per pass
 bool enqueue_kq_rows(uint8_t const* blocks, __half const* x, float* out, int const* offsets, int n, int bpr, int experts, int rows,
