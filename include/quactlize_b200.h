@@ -91,7 +91,8 @@ int quactlize_b200_vecdot_dev_v1(uint8_t const* blocks, int64_t block_bytes, uin
 int quactlize_b200_vecdot_moe_dev_v1(uint8_t const* blocks, int64_t block_bytes, uint16_t const* x, int const* offsets,
                                      float* out, int n, int blocks_per_row, int experts, int total_rows, int max_rows,
                                      int qtype, void* stream);
-/* in bounds whatever `offsets` hold: may be enqueued before they are checked; 40 = not covered, use the entry above */
+/* in bounds whatever `offsets` hold (clamped to [0, total_rows], none below the one before): may be enqueued before they are
+ * checked; 40 = not covered, use the entry above */
 int quactlize_b200_vecdot_moe_clamped_dev_v1(uint8_t const* blocks, int64_t block_bytes, uint16_t const* x, int const* offsets,
                                              float* out, int n, int blocks_per_row, int experts, int total_rows, int qtype,
                                              void* stream);

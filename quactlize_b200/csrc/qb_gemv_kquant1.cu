@@ -1,7 +1,7 @@
-// Raw-block decode GEMV for the four k-quant formats beside Q4_K (Q2_K, Q3_K, Q5_K, Q6_K), one activation row per
-// (expert, row): the copy structure of the Q4_K single-row kernel with a decode per format.
+// Dense raw-block decode GEMV for the four k-quant formats beside Q4_K (Q2_K, Q3_K, Q5_K, Q6_K), one activation row per pass
+// over the weights: the copy structure of the Q4_K single-row kernel with a decode per format.
 //
-//   out[t, r] = sum_k x[t, k] * W[r, k],   W = raw blocks [E][n][k/256][84|110|176|210] row-major by output row.
+//   out[t, r] = sum_k x[t, k] * W[r, k],   W = raw blocks [n][k/256][84|110|176|210] row-major by output row.
 //
 // Same contract as vecdot_rows_kernel of the reference for these formats (quactlize/include/gguf_vecdot.hpp:604-760, one
 // template over the five formats there too; bit meaning quactlize/include/gguf_vecdot.hpp:66-281).
@@ -22,7 +22,7 @@
 //
 // Blocks of 84, 110 and 210 bytes are only 4- or 2-byte aligned in a row: code runs are read as aligned words and, for the
 // 2-byte case, funnel-shifted by the lane's misalignment.  A K segment that does not start on a 16-byte boundary is
-// copied from the boundary below it (the row itself must be a multiple of 16 bytes, else the caller uses the plain kernel).
+// copied from the boundary below it (the row itself must be a multiple of 16 bytes, else the caller uses the several-row kernel).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 

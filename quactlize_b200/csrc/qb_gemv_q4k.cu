@@ -1,6 +1,6 @@
-// Q4_K decode GEMV, one activation row per (expert, row) -- the headline kernel.
+// Dense Q4_K decode GEMV, one activation row per pass over the weights -- the headline kernel.
 //
-//   out[t, r] = sum_k x[t, k] * W[r, k],   W = raw Q4_K blocks [E][n][k/256][144] row-major by output row.
+//   out[t, r] = sum_k x[t, k] * W[r, k],   W = raw Q4_K blocks [n][k/256][144] row-major by output row.
 //
 // Same contract as vecdot_rows_kernel of the reference (quactlize/include/gguf_vecdot.hpp:604-760, launch policy
 // quactlize/csrc/device/ppu_backend.cu:52-131) for Q4_K with a shared activation.

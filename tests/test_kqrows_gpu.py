@@ -114,6 +114,23 @@ def test_moe_takes_one_kernel_whoever_asks(qt, e, n, k, rows):
     assert kq.max_rel(native.cpu().numpy(), kq.vecdot_moe(blocks, x, off, n, k, qt)) < 2e-5
 
 
+@pytest.mark.parametrize("qt,m,n,k", [(12, 4, 600, 14336), (14, 8, 300, 4096)])
+def test_captured_launch(qt, m, n, k):
+    """A cluster launch and a plain one, captured with their plan already made and replayed on other activations."""
+    blocks = synth.kquant_blocks(qt, n * k // 256, seed=qt)
+    b, x = _cuda(blocks), _cuda(synth.activations(m, k, seed=1))
+    qb.gguf_vecdot_rows(b, x, n, k, qt)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = qb.gguf_vecdot_rows(b, x, n, k, qt)
+    for seed in (2, 3):
+        x.copy_(_cuda(synth.activations(m, k, seed=seed)))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, qb.gguf_vecdot_rows(b, x, n, k, qt))
+
+
 def test_moe_refuses_bad_offsets():
     """Offsets that do not describe the rows raise, whatever was enqueued meanwhile, and the next call is right."""
     e, n, k = 3, 64, 1024
