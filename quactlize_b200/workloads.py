@@ -258,7 +258,7 @@ def cfg5(bits: int, which: str, tokens: int, dev="cuda:0", run: Optional[Callabl
                     2.0 * rows * n * k, nb, launch, sample, "mixed_gemm_kernel (split-K) + splitk_reduce_kernel",
                     {"rows": rows, "active_experts_mean": round(act, 1), "banks": nb, "scale_zero_bytes": int(act * sz_expert)})
     return Case(f"cfg5_w{bits}a16_{which}_t{tokens}", "hbm", wb, int(act * (per_expert + sz_expert)) + rows * k * 2 + rows * n * 2,
-                2.0 * rows * n * k, nb, launch, sample, "rowmma_gemv_kernel",
+                2.0 * rows * n * k, nb, launch, sample, "rowmma_gemv_kernel" if rows >= 2 * e else "rowthread_gemv_kernel",
                 {"rows": rows, "active_experts_mean": round(act, 1), "banks": nb, "scale_zero_bytes": int(act * sz_expert)})
 
 
