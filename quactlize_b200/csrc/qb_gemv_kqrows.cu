@@ -18,8 +18,9 @@
 // fields, so an fp16 subnormal costs the sum as many bits as it has leading zeros.  The sub-scales therefore carry a power of two
 // (kr_up) that lifts the products out of the subnormals, a chain of MMAs is at most four long before its sum goes to a rounded
 // add, and a tile's K slices are added even and odd apart.  Relative error against 64 bits, N(0,1) activations, K 1280 to
-// 14336, against 22-bit group sums, chains of eight (Q6_K sixteen) and no lift: Q2_K 2.2e-7 -> 0.8e-7, Q3_K 1.2e-7 -> 0.8e-7, Q4_K 1.8e-7 ->
-// 1.2e-7, Q5_K 2.0e-7 -> 1.3e-7; 4096 -> 14336, us: Q2_K 8 rows 14.9 -> 13.1, Q3_K 4 rows 15.9 -> 16.2, Q4_K 8 rows 13.2 -> 13.0, Q5_K 4 rows 16.3 -> 16.2.  Q6_K, two products a code, has its chains cut only where a rounded kernel
+// 14336, against 22-bit group sums, chains of eight (Q6_K sixteen) and no lift: Q2_K 2.2e-7 -> 0.8e-7, Q3_K 1.2e-7 -> 0.8e-7,
+// Q4_K 1.8e-7 -> 1.2e-7, Q5_K 2.0e-7 -> 1.3e-7; 4096 -> 14336, us: Q2_K 8 rows 14.9 -> 13.1, Q3_K 4 rows 15.9 -> 16.2, Q4_K 8 rows
+// 13.2 -> 13.0, Q5_K 4 rows 16.3 -> 16.2.  Q6_K, two products a code, has its chains cut only where a rounded kernel
 // was before it: rows off a 16-byte boundary 2.3e-7 -> 1.0e-7 (4096 x 2304, three rows 8.0 -> 9.0 us; the plain kernel 0.8e-7 and 38 us);
 // its other rows took the one-row kernel's 8e-4 before and keep 2.3e-7.
 //
@@ -34,8 +35,8 @@
 // Rows of 84-, 110- and 210-byte blocks are read in 4-byte words, the word order rotated by the lane's quarter: rows lie
 // 16 bytes off a 128-byte pitch, so the 32 lanes of a load fall on 32 banks.  Every wait is bounded.
 //
-// Measured, 4096 -> 14336, eight rows, us: Q4_K 15.5 -> 13.4 (33 MB, 2.5 TB/s), Q2_K 41 -> 14.8, Q3_K 64 -> 16.6, Q5_K 58 -> 15.9,
-// Q6_K 66 -> 19.6.  What bounds it is the latency of a tile round, 1.13 us for Q4_K against 0.83 us of stream: about 260
+// Measured, 4096 -> 14336, eight rows, us: Q4_K 15.5 -> 13.0 (33 MB, 2.6 TB/s), Q2_K 41 -> 13.1, Q3_K 64 -> 16.4, Q5_K 58 -> 16.6,
+// Q6_K 66 -> 19.7.  What bounds it is the latency of a tile round, about 1.1 us for Q4_K against 0.83 us of stream: about 260
 // instructions a warp, half of them on the half-rate integer pipe, with four to five warps per scheduler.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -63,7 +64,7 @@ constexpr int kKrMaxStages = 8;
 constexpr int kKrMaxExperts = 4096;                // their offsets and group counts: 32 KB of shared memory at most
 constexpr int kKrAccTiles = 16;                    // tiles whose sums the reducing warp carries over K passes and CTAs
 // The first activations of a CTA by plain loads of the computing warps: 0.3 us earlier than through shared memory at one to
-// four rows (Q4_K 2400 x 4096, 2 rows: 6.05 against 6.43 us), later at eight (14336 x 4096: 14.1 against 13.4 us).
+// four rows (Q4_K 2400 x 4096, 2 rows: 6.05 against 6.43 us), later at eight (14336 x 4096: 13.3 against 12.9 us).
 constexpr int kKrDirectRows = 4;
 constexpr size_t kKrSmem = 227 * 1024;
 
