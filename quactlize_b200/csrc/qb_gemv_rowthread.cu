@@ -343,12 +343,15 @@ rowthread_gemv_kernel(const __grid_constant__ CUtensorMap map_lo, const __grid_c
     mbar_init_fence();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  // No griddepcontrol.launch_dependents: the next launch may start as this one's CTAs end (the trigger their exit implies).  Triggered
-  // here, its CTAs took the SMs this launch leaves idle and waited there through the whole kernel, and launches that arrive back to
-  // back took longer: W2 gs 64, 128 experts, 64 routed rows, 1536 x 2048 19.7 us a call with the trigger here, 18.2 with it after the
-  // main loop, 18.4 without; W4 gs 128 4096 x 4096 5.1, 5.0, 4.8; the same launches from a graph 18.2-18.4 and 4.8 in all three.
+  // Dependents start when a warp's last tile is requested (at once where the ring holds them all).  Triggered at the start of the stream,
+  // the next launch's CTAs took the SMs this launch leaves idle and waited there through the whole kernel, and launches that arrive back
+  // to back took longer: W2 gs 64, 128 experts, 64 routed rows, 1536 x 2048 19.7 us a call with the trigger at the start, 18.4 here, 18.2 after
+  // the main loop, 18.4 with none; from a graph 18.2-18.4 in all four.  Short launches from a graph want it early: W2 2048 x 768, one
+  // token 4.9 us, 5.15 with none.
+  auto dependents = [] { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); };
   auto start_stream = [&]() {
     for (int q = 0; q < STAGES && q < ntiles; ++q) issue(q);
+    if (ntiles <= STAGES) dependents();
   };
   if (nrows == 1) start_stream();
   for (int i = threadIdx.x; i < (nb_c + 16) * MR * TR; i += blockDim.x) part[i] = 0.f;
@@ -490,6 +493,7 @@ rowthread_gemv_kernel(const __grid_constant__ CUtensorMap map_lo, const __grid_c
       asm volatile("mov.u32 %0, %1;" : "=r"(sink) : "r"(dep) : "memory");
       __syncwarp();
       if (q + STAGES < ntiles) issue(q + STAGES);
+      if (q + STAGES + 1 == ntiles) dependents();
     }
     // scale channel of this lane's NQ runs, decoded once for all activation rows: weight = sv * (code + off) + zv
     float sv[WR][NQ], oz[WR][NQ];                            // scale, and (code offset * scale + zero)
